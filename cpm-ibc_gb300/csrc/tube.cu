@@ -180,6 +180,17 @@ __device__ void cp_segment(const double *pt, const double *a, const double *b, d
     for (int d = 0; d < 3; ++d) out[d] = a[d] + t * ab[d];
 }
 
+// closest point of x on primitive p (a triangle or a segment)
+__device__ __forceinline__ void closest_on_prim(const SurfaceParams &s, int64_t p, const double x[3], double q[3]) {
+    if (s.kind == CPM_TRIANGULATION) {
+        const int32_t *f = s.prims + 3 * p;
+        cp_triangle(x, s.verts + 3 * f[0], s.verts + 3 * f[1], s.verts + 3 * f[2], q);
+    } else {
+        const int32_t *f = s.prims + 2 * p;
+        cp_segment(x, s.verts + 3 * f[0], s.verts + 3 * f[1], q);
+    }
+}
+
 // Nearest mesh primitive through the uniform cell grid: rings of cells (by
 // Chebyshev distance) around the cell of x clamped into the grid box, until
 // the best distance is below the reach of the unsearched cells.  For y in the
@@ -189,7 +200,6 @@ __device__ void cp_segment(const double *pt, const double *a, const double *b, d
 // stops once nothing within max_dist can remain and reports dist > max_dist;
 // max_dist = +inf scans every primitive.
 __device__ void cp_mesh(const SurfaceParams &s, const double x[3], double cp[3], double &dist, double max_dist) {
-    const bool tri = s.kind == CPM_TRIANGULATION;
     double best2 = 1e300;
     int64_t bestp = -1;
     double bestcp[3] = {0, 0, 0};
@@ -201,13 +211,7 @@ __device__ void cp_mesh(const SurfaceParams &s, const double x[3], double cp[3],
     }
     auto test = [&](int64_t p) {
         double q[3];
-        if (tri) {
-            const int32_t *f = s.prims + 3 * p;
-            cp_triangle(x, s.verts + 3 * f[0], s.verts + 3 * f[1], s.verts + 3 * f[2], q);
-        } else {
-            const int32_t *f = s.prims + 2 * p;
-            cp_segment(x, s.verts + 3 * f[0], s.verts + 3 * f[1], q);
-        }
+        closest_on_prim(s, p, x, q);
         double dd[3] = {x[0] - q[0], x[1] - q[1], x[2] - q[2]};
         double d2 = dot3(dd, dd);
         if (d2 < best2 || (d2 == best2 && p < bestp)) {
@@ -739,10 +743,63 @@ static int tube_common_setup(cpm_tube_s *t, const cpm_surface_desc *d, int32_t p
 }
 
 // FindStartingPoint (src/Tube.cpp:540-551): cp of the xstart corner, rounded.
-__global__ void k_seed(SurfaceParams s, GridParams g, int32_t *seed) {
-    double x[3] = {g.xstart, g.xstart, g.xstart}, cp[3], d;
-    closest_point(s, x, cp, d);
+// The corner is far from the surface, so a mesh is scanned whole: by SEED_BLOCKS
+// blocks, each leaving its nearest primitive (the lower index of equally near
+// ones, as cp_mesh has it), and one warp picks among them.  One thread scanning
+// 20,480 triangles took 125 of the 142 ms of a tube build.
+constexpr int SEED_T = 256, SEED_BLOCKS = 128;
+struct SeedBest {
+    double d2, cp[3];
+    long long prim;  // -1: none
+};
+__device__ __forceinline__ bool seed_less(double d2, long long p, const SeedBest &b) {
+    return p >= 0 && (b.prim < 0 || d2 < b.d2 || (d2 == b.d2 && p < b.prim));
+}
+__global__ void __launch_bounds__(SEED_T) k_seed_mesh(SurfaceParams s, GridParams g, SeedBest *__restrict__ best) {
+    __shared__ SeedBest sh[SEED_T];
+    const double x[3] = {g.xstart, g.xstart, g.xstart};
+    SeedBest b{1e300, {0, 0, 0}, -1};
+    for (long long p = (long long)blockIdx.x * SEED_T + threadIdx.x; p < s.nprims; p += (long long)gridDim.x * SEED_T) {
+        double q[3];
+        closest_on_prim(s, p, x, q);
+        const double dd[3] = {x[0] - q[0], x[1] - q[1], x[2] - q[2]}, d2 = dot3(dd, dd);
+        if (d2 < 1e300 && seed_less(d2, p, b)) b = SeedBest{d2, {q[0], q[1], q[2]}, p};
+    }
+    sh[threadIdx.x] = b;
+    __syncthreads();
+    for (int h = SEED_T / 2; h > 0; h >>= 1) {
+        if (threadIdx.x < h && seed_less(sh[threadIdx.x + h].d2, sh[threadIdx.x + h].prim, sh[threadIdx.x]))
+            sh[threadIdx.x] = sh[threadIdx.x + h];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) best[blockIdx.x] = sh[0];
+}
+__global__ void k_seed(SurfaceParams s, GridParams g, const SeedBest *__restrict__ best, int32_t *seed) {
+    double x[3] = {g.xstart, g.xstart, g.xstart}, cp[3] = {0, 0, 0}, d;
+    if (best) {
+        SeedBest b{1e300, {0, 0, 0}, -1};
+        for (int i = 0; i < SEED_BLOCKS; ++i)
+            if (seed_less(best[i].d2, best[i].prim, b)) b = best[i];
+        for (int k = 0; k < 3; ++k) cp[k] = b.cp[k];
+    } else {
+        closest_point(s, x, cp, d);
+    }
     for (int k = 0; k < 3; ++k) seed[k] = (int32_t)round((cp[k] - g.xstart) / g.dx);
+}
+
+// the tube's seed node, into host memory (waits)
+static int find_seed(const SurfaceParams &sp, const GridParams &g, std::vector<int32_t> &sh) {
+    DBuf<int32_t> seed;
+    DBuf<SeedBest> best;
+    CPM_TRY(seed.alloc(3));
+    const bool mesh = sp.kind == CPM_TRIANGULATION || sp.kind == CPM_POLYLINE;
+    if (mesh) {
+        CPM_TRY(best.alloc(SEED_BLOCKS));
+        k_seed_mesh<<<SEED_BLOCKS, SEED_T, 0, stream()>>>(sp, g, best.p);
+    }
+    k_seed<<<1, 1, 0, stream()>>>(sp, g, mesh ? best.p : nullptr, seed.p);
+    CPM_CUDA_TRY(cudaGetLastError());
+    return seed.download(sh, 3);
 }
 
 }  // namespace cpm
@@ -763,14 +820,13 @@ extern "C" int cpm_tube_build(const cpm_surface_desc *surface, int32_t p, double
     SurfaceParams sp = t->surf.params();
     const int bs = 256;
     int64_t nb3 = (int64_t)g.NB * g.NB * g.NB;
-    DBuf<int32_t> flag, seed;
-    if ((rc = flag.alloc(nb3)) || (rc = seed.alloc(3))) return bail(rc);
+    DBuf<int32_t> flag;
+    if ((rc = flag.alloc(nb3))) return bail(rc);
     double thresh = g.radius + g.dx + 1.5 * std::sqrt(3.0) * g.dx + 1e-9 * (1.0 + g.radius);
     k_brick_candidates<<<(unsigned)((nb3 + bs - 1) / bs), bs, 0, stream()>>>(sp, g, thresh, flag.p);
-    k_seed<<<1, 1, 0, stream()>>>(sp, g, seed.p);
     if (cudaGetLastError() != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "candidate kernel launch failed"));
     std::vector<int32_t> fh, sh;
-    if ((rc = flag.download(fh, nb3)) || (rc = seed.download(sh, 3))) return bail(rc);
+    if ((rc = find_seed(sp, g, sh)) || (rc = flag.download(fh, nb3))) return bail(rc);
     std::vector<uint32_t> cand_h;
     std::vector<int32_t> cmap_h((size_t)nb3, -1);
     for (int64_t b = 0; b < nb3; ++b)
@@ -833,11 +889,8 @@ extern "C" int cpm_tube_build_from_cp(const cpm_surface_desc *surface, int32_t p
     }
     // seed from the supplied closest point of the xstart corner is not available:
     // use the device closest point of the corner, as cpm_tube_build does.
-    DBuf<int32_t> seed;
-    if ((rc = seed.alloc(3))) return bail(rc);
-    k_seed<<<1, 1, 0, stream()>>>(t->surf.params(), g, seed.p);
     std::vector<int32_t> sh;
-    if ((rc = seed.download(sh, 3))) return bail(rc);
+    if ((rc = find_seed(t->surf.params(), g, sh))) return bail(rc);
     DBuf<uint32_t> cand;
     DBuf<double> ccp, cdist;
     DBuf<uint8_t> band;
