@@ -25,7 +25,7 @@ namespace cpm {
 
 template <class T>
 static OpView<T> make_view(const cpm_opset_s *o, const T *w, const T *xval, const T *lval, const T *ldiag, const T *w_ord,
-                           const T *pl_xval, const T *pe_w, const T *sp_w, const T *ov_w) {
+                           const T *sp_w, const T *ov_w) {
     OpView<T> v;
     v.bv = o->tube->view();
     v.N = o->N;
@@ -55,19 +55,14 @@ static OpView<T> make_view(const cpm_opset_s *o, const T *w, const T *xval, cons
     v.ident = o->ident.p;
     v.gcols = o->gcols.p;
     v.w_ord = w_ord;
+    v.w_fix = o->w_fix.p;
+    v.chunk = o->chunk.p;
+    v.n_chunk = o->n_chunk;
     v.fl_ord = o->fl_ord.p;
     v.n_ord = o->n_ord;
     v.n_grp = o->n_grp;
+    v.n_grp_plain = o->n_grp_plain;
     v.n_ident = o->n_ident;
-    v.pl_row = o->pl_row.p;
-    v.pl_off = o->pl_off.p;
-    v.pl_xcol = o->pl_xcol.p;
-    v.pl_neg = o->pl_neg.p;
-    v.pl_xval = pl_xval;
-    v.pe_new = o->pe_new.p;
-    v.pe_old = o->pe_old.p;
-    v.pe_w = pe_w;
-    v.n_pl = o->n_pl;
     v.n_sp_rows = o->n_sp_rows;
     v.e32_bps = o->e32_bps;
     v.patch_bps = o->patch_bps;
@@ -86,11 +81,11 @@ static OpView<T> make_view(const cpm_opset_s *o, const T *w, const T *xval, cons
 
 template <>
 cpm::OpView<double> cpm_opset_s::view<double>() const {
-    return cpm::make_view<double>(this, w.p, p_xval.p, lval.p, ldiag.p, w_ord.p, pl_xval.p, pe_w.p, sp_w.p, ov_w.p);
+    return cpm::make_view<double>(this, w.p, p_xval.p, lval.p, ldiag.p, w_ord.p, sp_w.p, ov_w.p);
 }
 template <>
 cpm::OpView<float> cpm_opset_s::view<float>() const {
-    return cpm::make_view<float>(this, w32.p, p_xval32.p, lval32.p, ldiag32.p, w_ord32.p, pl_xval32.p, pe_w32.p, sp_w32.p, ov_w32.p);
+    return cpm::make_view<float>(this, w32.p, p_xval32.p, lval32.p, ldiag32.p, w_ord32.p, sp_w32.p, ov_w32.p);
 }
 
 namespace cpm {
@@ -1186,8 +1181,6 @@ static int make_float_copies(cpm_opset_s *o) {
     CPM_TRY(conv(o->p_xval, o->p_xval32));
     CPM_TRY(conv(o->lval, o->lval32));
     CPM_TRY(conv(o->ldiag, o->ldiag32));
-    CPM_TRY(conv(o->pl_xval, o->pl_xval32));
-    CPM_TRY(conv(o->pe_w, o->pe_w32));
     if (o->ov_w.n) CPM_TRY(conv(o->ov_w, o->ov_w32));
     return 0;
 }
@@ -1623,117 +1616,41 @@ __global__ void k_build_nbr6_ibc(OpView<double> op, int32_t *__restrict__ nbr6, 
     for (int d = 0; d < 6; ++d) nbr6[6 * r + d] = (!ident && e0 + d < e1) ? op.lcol[e0 + d] : -1;
 }
 
-// 64 bulk stencil columns of each base group (s = 16 i + 4 j + k)
+// the 64 columns of each group, moves applied (the same in all rows of the group)
 __global__ void k_group_cols(OpView<double> op, int64_t n_grp, int32_t *__restrict__ gcols) {
     int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= 64 * n_grp) return;
     int64_t g = e >> 6;
     int s = (int)(e & 63);
-    uint32_t b = op.base[op.ord[op.grp[g]]];
+    const int r = op.ord[op.grp[g]];
+    if (g >= op.n_grp_plain) {
+        const int pi = op.patch[r];
+        const uint64_t em = op.p_emask[pi];
+        if ((em >> s) & 1ull) {
+            gcols[e] = op.moved[op.p_eoff[pi] + __popcll(em & ((1ull << s) - 1ull))];
+            return;
+        }
+    }
+    uint32_t b = op.base[r];
     int col = node_at(op.bv, unpack_i(b) + (s >> 4), unpack_j(b) + ((s >> 2) & 3), unpack_k(b) + (s & 3));
     gcols[e] = col >= 0 ? col : 0;  // missing stencil nodes are rejected at tube build time
 }
 
-// weights and flags in base-sorted row order
-__global__ void k_sorted_rows(OpView<double> op, int64_t n_ord, double *__restrict__ w_ord, uint8_t *__restrict__ fl_ord) {
+// weights (FP64 and fixed point) and flags in group order
+__global__ void k_sorted_rows(OpView<double> op, int64_t n_ord, double *__restrict__ w_ord, int2 *__restrict__ w_fix,
+                              uint8_t *__restrict__ fl_ord) {
     int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= 12 * n_ord) return;
     int64_t p = e / 12;
     int a = (int)(e % 12);
     int64_t r = op.ord[p];
     w_ord[e] = op.w[12 * r + a];
+    w_fix[e] = fx_weight(op.w[12 * r + a]);
     if (a == 0) fl_ord[p] = op.flags[r];
 }
 
-// entries of the patch list: one thread per patched row, moved points in
-// increasing stencil order s = 16 i + 4 j + k
-__global__ void k_patch_entries(OpView<double> op, int64_t n_pl, int32_t *__restrict__ pe_new, int32_t *__restrict__ pe_old,
-                                double *__restrict__ pe_w, int *__restrict__ err) {
-    int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (q >= n_pl) return;
-    const int r = op.pl_row[q];
-    const int pi = op.patch[r];
-    uint64_t em = (op.flags[r] & F_EMOVE) ? op.p_emask[pi] : 0ull;
-    int mo = op.p_eoff[pi];
-    const uint32_t b = op.base[r];
-    const int bi = unpack_i(b), bj = unpack_j(b), bk = unpack_k(b);
-    const double *w = op.w + 12 * (int64_t)r;
-    int e = op.pl_off[q];
-    while (em) {
-        const int s = __ffsll((long long)em) - 1;
-        em &= em - 1;
-        const int i = s >> 4, j = (s >> 2) & 3, k = s & 3;
-        const int old = node_at(op.bv, bi + i, bj + j, bk + k);
-        if (old < 0) atomicOr(err, 1);
-        pe_new[e] = op.moved[mo++];
-        pe_old[e] = old < 0 ? 0 : old;
-        pe_w[e] = (w[i] * w[4 + j]) * w[8 + k];
-        ++e;
-    }
-}
-
-// The patch list: rows whose E row is not the plain bulk stencil (moved
-// columns, negation, an extra entry), so the 32-slot E passes can evaluate
-// every row as bulk and correct these rows in a separate, parallel pass.
-static int build_patch_list(cpm_opset_s *o, const std::vector<uint8_t> &flags) {
-    const int64_t D = o->D;
-    std::vector<int32_t> patch, p_xcol;
-    std::vector<uint64_t> p_emask;
-    std::vector<double> p_xval;
-    std::vector<int32_t> rows, off{0}, xcol;
-    std::vector<uint8_t> neg;
-    std::vector<double> xval;
-    if (o->patch.n >= (size_t)D) {
-        CPM_TRY(o->patch.download(patch, D));
-        CPM_TRY(o->p_emask.download(p_emask, o->p_emask.n));
-        CPM_TRY(o->p_xcol.download(p_xcol, o->p_xcol.n));
-        CPM_TRY(o->p_xval.download(p_xval, o->p_xval.n));
-        for (int64_t r = 0; r < D; ++r) {
-            const uint8_t f = flags[r];
-            if ((f & F_IDENT) || !(f & (F_EMOVE | F_EXTRA | F_ENEG))) continue;
-            const int pi = patch[r];
-            if (pi < 0 || (size_t)pi >= p_emask.size()) return fail(CPM_ERR_CUDA, "internal: patched row without a patch record");
-            rows.push_back((int32_t)r);
-            off.push_back(off.back() + ((f & F_EMOVE) ? __builtin_popcountll(p_emask[pi]) : 0));
-            const bool ex = (f & F_OVL) && o->h_ov_ptr[2 * pi + 1] > o->h_ov_ptr[2 * pi];
-            neg.push_back((uint8_t)(((f & F_ENEG) ? 1 : 0) | (ex ? 2 : 0)));
-            xcol.push_back((f & F_EXTRA) ? p_xcol[pi] : -1);
-            xval.push_back((f & F_EXTRA) ? p_xval[pi] : 0.0);
-        }
-    }
-    o->n_pl = (int64_t)rows.size();
-    const int64_t ne = off.back();
-    o->n_pe = ne;
-    if (rows.empty()) {
-        rows.push_back(0);
-        neg.push_back(0);
-        xcol.push_back(-1);
-        xval.push_back(0.0);
-    }
-    CPM_TRY(o->pl_row.upload(rows));
-    CPM_TRY(o->pl_off.upload(off));
-    CPM_TRY(o->pl_neg.upload(neg));
-    CPM_TRY(o->pl_xcol.upload(xcol));
-    CPM_TRY(o->pl_xval.upload(xval));
-    CPM_TRY(o->pe_new.alloc(std::max<int64_t>(1, ne)));
-    CPM_TRY(o->pe_old.alloc(std::max<int64_t>(1, ne)));
-    CPM_TRY(o->pe_w.alloc(std::max<int64_t>(1, ne)));
-    if (o->n_pl > 0) {
-        DBuf<int> err;
-        CPM_TRY(err.alloc(1));
-        CPM_TRY(err.zero());
-        k_patch_entries<<<(unsigned)((o->n_pl + 255) / 256), 256, 0, stream()>>>(o->view<double>(), o->n_pl, o->pe_new.p,
-                                                                                 o->pe_old.p, o->pe_w.p, err.p);
-        CPM_CUDA_TRY(cudaGetLastError());
-        std::vector<int> he;
-        CPM_TRY(err.download(he, 1));
-        if (he[0]) return fail(CPM_ERR_CUDA, "internal: a moved stencil point has no tube node");
-    }
-    return 0;
-}
-
-// Apply schedule: neighbour table, rows sorted by base point with their groups,
-// identity rows.  Rows sharing a base point read the same 64 values of x.
+// Apply schedule: neighbour table, groups of rows that read the same 64 values
+// of x, identity rows.
 static int build_schedule(cpm_opset_s *o) {
     const int64_t N = o->N, D = o->D;
     CPM_TRY(o->nbr6.alloc(6 * D));
@@ -1753,22 +1670,82 @@ static int build_schedule(cpm_opset_s *o) {
     std::vector<uint32_t> base;
     CPM_TRY(o->flags.download(flags, D));
     CPM_TRY(o->base.download(base, D));
-    std::vector<std::pair<uint32_t, int32_t>> rows;
+    std::vector<int32_t> patch, p_eoff, moved;
+    std::vector<uint64_t> p_emask;
+    if (o->patch.n >= (size_t)D) {
+        CPM_TRY(o->patch.download(patch, D));
+        CPM_TRY(o->p_emask.download(p_emask, o->p_emask.n));
+        CPM_TRY(o->p_eoff.download(p_eoff, o->p_eoff.n));
+        CPM_TRY(o->moved.download(moved, o->moved.n));
+    }
+    std::vector<uint64_t> rows;  // rows without moved columns: base point << 32 | row
+    std::vector<std::pair<uint32_t, int32_t>> crossing;  // and with
     std::vector<int32_t> ident;
     rows.reserve(D);
+    o->n_pl = o->n_pe = 0;
     for (int64_t r = 0; r < D; ++r) {
-        if (flags[r] & F_IDENT)
+        const uint8_t f = flags[r];
+        if (f & F_IDENT) {
             ident.push_back((int32_t)r);
-        else
-            rows.push_back({base[r], (int32_t)r});
+            continue;
+        }
+        if (f & (F_EMOVE | F_EXTRA | F_ENEG)) {
+            if (patch.empty() || patch[r] < 0 || (size_t)patch[r] >= p_emask.size())
+                return fail(CPM_ERR_CUDA, "internal: patched row without a patch record");
+            ++o->n_pl;
+        }
+        if ((f & F_EMOVE) && p_emask[patch[r]]) {
+            o->n_pe += __builtin_popcountll(p_emask[patch[r]]);
+            crossing.push_back({base[r], (int32_t)r});
+        } else {
+            rows.push_back((uint64_t)base[r] << 32 | (uint64_t)r);
+        }
     }
     std::sort(rows.begin(), rows.end());
-    std::vector<int32_t> ord(rows.size()), grp;
+    std::vector<int32_t> ord, grp;
+    ord.reserve(rows.size() + crossing.size());
     for (size_t p = 0; p < rows.size(); ++p) {
-        ord[p] = rows[p].second;
-        if (p == 0 || rows[p].first != rows[p - 1].first) grp.push_back((int32_t)p);
+        ord.push_back((int32_t)(uint32_t)rows[p]);
+        if (p == 0 || rows[p] >> 32 != rows[p - 1] >> 32) grp.push_back((int32_t)p);
     }
-    grp.push_back((int32_t)rows.size());
+    o->n_grp_plain = (int64_t)grp.size();
+    // -1, 0, 1: order of two crossing rows by base point, moved points and their columns
+    auto order = [&](const std::pair<uint32_t, int32_t> &a, const std::pair<uint32_t, int32_t> &b) -> int {
+        if (a.first != b.first) return a.first < b.first ? -1 : 1;
+        const int pa = patch[a.second], pb = patch[b.second];
+        if (p_emask[pa] != p_emask[pb]) return p_emask[pa] < p_emask[pb] ? -1 : 1;
+        const int n = __builtin_popcountll(p_emask[pa]);
+        for (int e = 0; e < n; ++e) {
+            const int32_t ca = moved[p_eoff[pa] + e], cb = moved[p_eoff[pb] + e];
+            if (ca != cb) return ca < cb ? -1 : 1;
+        }
+        return 0;
+    };
+    std::sort(crossing.begin(), crossing.end(), [&](const std::pair<uint32_t, int32_t> &a, const std::pair<uint32_t, int32_t> &b) {
+        const int c = order(a, b);
+        return c ? c < 0 : a.second < b.second;
+    });
+    for (size_t p = 0; p < crossing.size(); ++p) {
+        if (p == 0 || order(crossing[p - 1], crossing[p])) grp.push_back((int32_t)ord.size());
+        ord.push_back(crossing[p].second);
+    }
+    grp.push_back((int32_t)ord.size());
+    std::vector<int4> chunk;
+    for (size_t g = 0; g + 1 < grp.size();) {
+        int4 c = make_int4((int)g, chunk.empty() ? 0 : chunk.back().y + (chunk.back().w & 255), 1, 0);
+        int rows_c = 0, groups_c = 0;
+        while (g + 1 < grp.size() && rows_c < 32 && groups_c < E1_GROUPS) {
+            c.z |= (int)(1u << rows_c);
+            ++groups_c;
+            rows_c = std::min(32, grp[g + 1] - c.y);
+            if (grp[g + 1] - c.y > 32) break;  // the group goes on in the next run
+            ++g;
+        }
+        c.w = rows_c | groups_c << 8;
+        chunk.push_back(c);
+    }
+    o->n_chunk = (int64_t)chunk.size();
+    if (chunk.empty()) chunk.push_back(make_int4(0, 0, 0, 0));
     o->n_ord = (int64_t)ord.size();
     o->n_grp = (int64_t)grp.size() - 1;
     o->n_ident = (int64_t)ident.size();
@@ -1776,18 +1753,20 @@ static int build_schedule(cpm_opset_s *o) {
     if (ident.empty()) ident.push_back(0);
     CPM_TRY(o->ord.upload(ord));
     CPM_TRY(o->grp.upload(grp));
+    CPM_TRY(o->chunk.upload(chunk));
     CPM_TRY(o->ident.upload(ident));
-    // per group: its 64 bulk stencil columns; per sorted row: weights and flags
+    // per group: its 64 columns; per sorted row: weights and flags
     CPM_TRY(o->gcols.alloc(64 * std::max<int64_t>(1, o->n_grp)));
     CPM_TRY(o->w_ord.alloc(12 * std::max<int64_t>(1, o->n_ord)));
+    CPM_TRY(o->w_fix.alloc(12 * std::max<int64_t>(1, o->n_ord)));
     CPM_TRY(o->fl_ord.alloc(std::max<int64_t>(1, o->n_ord)));
     if (o->n_grp > 0) {
         k_group_cols<<<(unsigned)((64 * o->n_grp + 255) / 256), 256, 0, stream()>>>(o->view<double>(), o->n_grp, o->gcols.p);
         k_sorted_rows<<<(unsigned)((12 * o->n_ord + 255) / 256), 256, 0, stream()>>>(o->view<double>(), o->n_ord, o->w_ord.p,
-                                                                                    o->fl_ord.p);
+                                                                                    o->w_fix.p, o->fl_ord.p);
         CPM_CUDA_TRY(cudaGetLastError());
     }
-    return build_patch_list(o, flags);
+    return 0;
 }
 
 }  // namespace cpm

@@ -5,6 +5,7 @@
 #include <memory>
 
 #include "cpm_internal.h"
+#include "fixed62.h"
 
 namespace cpm {
 
@@ -46,20 +47,19 @@ struct OpView {
     // apply schedule
     const int32_t *nbr6;    // D x 6: each row's L columns (moves applied, -1 absent); all rows'
                             // L rows are Ldiag on the diagonal and Loff off it
-    const int32_t *ord;     // non-identity rows sorted by base point (stable in row order)
-    const int32_t *grp;     // base groups: ord[grp[g] .. grp[g+1]) share one base point
-    const int32_t *gcols;   // 64 bulk stencil columns per group, s = 16 i + 4 j + k
+    // Groups: the non-identity rows that read the same 64 columns.  First the
+    // groups of rows without moved columns (one per base point, n_grp_plain of
+    // them, in base-point order), then those of rows whose stencil crosses an IBC
+    // (same base point and same moved columns).
+    const int32_t *ord;     // non-identity rows, group by group
+    const int32_t *grp;     // ord[grp[g] .. grp[g+1]) is group g
+    const int32_t *gcols;   // 64 columns per group, s = 16 i + 4 j + k, moves applied
     const T *w_ord;         // weights of ord[p] at 12 p (sorted copy: coalesced per group)
+    const int2 *w_fix;      // the same weights in fixed point (FP64 passes; fx_weight)
+    const int4 *chunk;      // one-vector pass: runs of ord (see E1_GROUPS)
     const uint8_t *fl_ord;  // flags of ord[p]
     const int32_t *ident;   // identity rows
-    // IBC patch list of the rows whose E row differs from the bulk stencil:
-    // t_r = sign (bulk + sum_e w_e (x[new_e] - x[old_e])) + xval x[xcol]
-    const int32_t *pl_row, *pl_off, *pl_xcol;  // n_pl rows; entries pl_off[i] .. pl_off[i+1]
-    const uint8_t *pl_neg;                    // bit 0: negated (2nd-order Dirichlet DOF rows); bit 1: E extras (F_OVL)
-    const T *pl_xval;
-    const int32_t *pe_new, *pe_old;           // moved column and the bulk column it replaces
-    const T *pe_w;                            // stencil weight (wx_i wy_j) wz_k of the moved point
-    int64_t n_ord, n_grp, n_ident, n_pl;
+    int64_t n_ord, n_grp, n_grp_plain, n_ident, n_chunk;
     // per-slot patches of a batch whose slots each carry their own point IBC
     // (cpm_geodesic_batch_*): row r's records sp_rec[sp_ptr[r] .. sp_ptr[r + 1]),
     // {slot, 0 E entry / 1 L entry, the column it replaces, the slot's DOF column};
@@ -279,20 +279,11 @@ __device__ __forceinline__ void load_w12(const double *w, double (&o)[12]) {
     }
 }
 
-// Four-warp-per-group E pass for a 32-slot batch (stencil split by planes).
-// Warp w holds the 16 nodes of plane i = w of the group's 4^3 stencil (lane =
-// slot), evaluates wx_w * sum_j wy_j sum_k wz_k x for every row of the group,
-// and the four planes are summed through shared memory.  16 registers per
-// plane instead of 64 keep ~4x more warps resident to hide gather latency.
-// Every row gets the bulk stencil; rows on the IBC patch list are corrected
-// afterwards (k_epatch32).
-constexpr int EG_ROWS = 32;  // rows per shared-memory chunk of a group
-template <class T>
-struct EGShared {
-    T part[4][EG_ROWS][32];
-    alignas(16) T w[EG_ROWS * 12];
-    int rows[EG_ROWS];
-};
+// a warp of the one-vector pass takes a run of at most 32 rows of at most E1_GROUPS
+// groups: {first group, first row p, bit l set where row p + l opens a group of
+// the run, rows | groups << 8}.  Groups without moved columns have 6 rows on
+// average, so eight nearly always fill a warp.
+constexpr int E1_GROUPS = 8;
 
 // packed FP32 pairs (f32x2 arithmetic, one instruction for two rows)
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
@@ -347,9 +338,9 @@ __device__ __forceinline__ void lds4(const double *p, double (&o)[4]) {
     o[3] = b.y;
 }
 
-// the 16 columns of plane `warp` of group g: four 16-byte loads every lane makes alike
-__device__ __forceinline__ void e_group_cols(const int32_t *gcols, int64_t g, int warp, int (&col)[16]) {
-    const int4 *gc = (const int4 *)(gcols + 64 * g + 16 * warp);
+// the 16 columns of plane `plane` of group g: four 16-byte loads every lane makes alike
+__device__ __forceinline__ void e_group_cols(const int32_t *gcols, int64_t g, int plane, int (&col)[16]) {
+    const int4 *gc = (const int4 *)(gcols + 64 * g + 16 * plane);
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
         const int4 c = __ldg(gc + v);
@@ -359,84 +350,17 @@ __device__ __forceinline__ void e_group_cols(const int32_t *gcols, int64_t g, in
         col[4 * v + 3] = c.w;
     }
 }
-// the plane's 16 x values of this lane's slot (inactive slots issue no memory requests)
-template <class T>
-__device__ __forceinline__ void e_group_x(const T *__restrict__ x, const int (&col)[16], int lane, bool act, T (&xb)[16]) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q) xb[q] = act ? x[(uint32_t)col[q] * 32u + lane] : T(0);
-}
-
-// rows ord[p0 .. p1) of group g from the plane's x values xb
-template <class T>
-__device__ __forceinline__ void e_group_split(const OpView<T> &op, int p0, int p1, int warp, int lane, bool act, EGShared<T> &sh,
-                                              const T (&xb)[16], T *__restrict__ t) {
-    const int tid = warp * 32 + lane;
-    for (int c0 = p0; c0 < p1; c0 += EG_ROWS) {
-        const int nr = min(p1 - c0, EG_ROWS);
-        if constexpr (sizeof(T) == 4) {
-            // FP32: rows in pairs with packed f32x2 arithmetic.  The chunk's weights
-            // are staged pair-interleaved (component c of rows 2p, 2p+1 at
-            // 24 p + 2 c, 24 p + 2 c + 1), zero for the odd row of a last pair.
-            const int nr2 = nr + (nr & 1);
-            for (int e = tid; e < nr2 * 12; e += 128) {
-                const int q = e / 12, c = e - 12 * q;
-                sh.w[24 * (q >> 1) + 2 * c + (q & 1)] = q < nr ? op.w_ord[12 * (size_t)(c0 + q) + c] : T(0);
-            }
-            if (tid < nr) sh.rows[tid] = op.ord[c0 + tid];
-            __syncthreads();
-            uint64_t x2[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) x2[q] = f2_pack((float)xb[q], (float)xb[q]);
-            for (int q = 0; q < nr; q += 2) {
-                const float *w = (const float *)sh.w + 12 * q;
-                const uint64_t wx2 = *(const uint64_t *)(w + 2 * warp);
-                const ulonglong2 y01 = *(const ulonglong2 *)(w + 8), y23 = *(const ulonglong2 *)(w + 12);
-                const ulonglong2 z01 = *(const ulonglong2 *)(w + 16), z23 = *(const ulonglong2 *)(w + 20);
-                const uint64_t wy2[4] = {y01.x, y01.y, y23.x, y23.y}, wz2[4] = {z01.x, z01.y, z23.x, z23.y};
-                uint64_t ay2 = 0ull;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint64_t az2 = f2_mul(wz2[0], x2[4 * j]);
-                    az2 = f2_fma(wz2[1], x2[4 * j + 1], az2);
-                    az2 = f2_fma(wz2[2], x2[4 * j + 2], az2);
-                    az2 = f2_fma(wz2[3], x2[4 * j + 3], az2);
-                    ay2 = j == 0 ? f2_mul(wy2[0], az2) : f2_fma(wy2[j], az2, ay2);
-                }
-                float lo, hi;
-                f2_unpack(f2_mul(wx2, ay2), lo, hi);
-                sh.part[warp][q][lane] = (T)lo;
-                if (q + 1 < nr) sh.part[warp][q + 1][lane] = (T)hi;
-            }
-        } else {
-        // stage the chunk's sorted weights, row ids and flags (coalesced, independent loads)
-        for (int e = tid; e < nr * 12; e += 128) sh.w[e] = op.w_ord[12 * (size_t)c0 + e];
-        if (tid < nr) sh.rows[tid] = op.ord[c0 + tid];
-        __syncthreads();
-        for (int q = 0; q < nr; ++q) {
-            const T *w = sh.w + 12 * q;
-            const T wxi = w[warp];
-            T wy[4], wz[4];
-            lds4(w + 4, wy);
-            lds4(w + 8, wz);
-            T ay = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                T az = 0;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) az += wz[k] * xb[4 * j + k];
-                ay += wy[j] * az;
-            }
-            sh.part[warp][q][lane] = wxi * ay;
-        }
-        }
-        __syncthreads();
-        for (int q = warp; q < nr; q += 4) {
-            const int r = sh.rows[q];
-            const T acc = ((sh.part[0][q][lane] + sh.part[1][q][lane]) + sh.part[2][q][lane]) + sh.part[3][q][lane];
-            if (act) t[(uint32_t)r * 32u + lane] = acc;
-        }
-        __syncthreads();
-    }
+// a row's terms beyond its 64 weighted values, from the sum acc of those: the
+// further copies of entries that lie across several IBCs, the sign of 2nd-order
+// Dirichlet DOF rows and their extra entry (slot s of a K-wide batch)
+constexpr uint8_t F_TERMS = F_OVL | F_ENEG | F_EXTRA;
+template <class T, int K>
+__device__ __forceinline__ T e_row_terms(const OpView<T> &op, uint8_t fl, int r, int s, T acc, const T *__restrict__ x) {
+    const int pi = op.patch[r];
+    if (fl & F_OVL) acc += ovl_e_sum<T, K>(op.ov_ptr, op.ov_col, op.ov_w, pi, s, x);
+    if (fl & F_ENEG) acc = -acc;
+    if (fl & F_EXTRA) acc += op.p_xval[pi] * x[(int64_t)op.p_xcol[pi] * K + s];
+    return acc;
 }
 
 // The extra L targets of an F_OVL row r (OpView::ov_*), added to a finished
@@ -605,15 +529,13 @@ struct cpm_opset_s {
     cpm::DBuf<double> p_xval, lval, ldiag;
     cpm::DBuf<float> p_xval32, lval32, ldiag32;
     cpm::DBuf<int32_t> nbr6, ord, grp, ident, gcols;
-    cpm::DBuf<int32_t> pl_row, pl_off, pl_xcol, pe_new, pe_old;
-    cpm::DBuf<uint8_t> pl_neg;
-    cpm::DBuf<double> pl_xval, pe_w;
-    cpm::DBuf<float> pl_xval32, pe_w32;
-    int64_t n_pl = 0, n_pe = 0;
+    int64_t n_pl = 0, n_pe = 0;  // rows whose E row is not the plain stencil; moved E stencil points
     cpm::DBuf<double> w_ord;
     cpm::DBuf<float> w_ord32;
+    cpm::DBuf<int2> w_fix;
+    cpm::DBuf<int4> chunk;
     cpm::DBuf<uint8_t> fl_ord;
-    int64_t n_ord = 0, n_grp = 0, n_ident = 0;
+    int64_t n_ord = 0, n_grp = 0, n_grp_plain = 0, n_ident = 0, n_chunk = 0;
     // host-side row layout for right-hand sides
     std::vector<uint8_t> h_identity;
     std::vector<int32_t> h_kind, h_ibc, h_side;

@@ -303,22 +303,24 @@ __device__ __forceinline__ void xr_update(Slot &S, const SolveParams &P, double 
 
 // ================================================================= kernels
 
-// 32 slots, plane-split: one 4-warp block per base group (grid-stride), then
-// identity rows copied warp per row.  ph < 0: every slot.
-template <class T>
-__global__ void __launch_bounds__(128) k_epass32s(OpView<T> op, const Slot *__restrict__ sl, int ph, const T *__restrict__ x,
-                                                  T *__restrict__ t) {
-    __shared__ EGShared<T> sh;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool act = (ph < 0) || sl[lane].phase == ph;
-    if (!__any_sync(FULL, act)) return;  // the same 32 slots in every warp: block-uniform
-    for (int64_t g = blockIdx.x; g < op.n_grp; g += gridDim.x) {
-        int col[16];
-        T xb[16];
-        e_group_cols(op.gcols, g, warp, col);
-        e_group_x(x, col, lane, act, xb);
-        e_group_split<T>(op, op.grp[g], op.grp[g + 1], warp, lane, act, sh, xb, t);
+// the groups of one warp of a 32-slot pass: blocks [0, nb_plain) stride over the
+// groups without moved columns, the others over the rest
+struct GroupLoop {
+    int64_t g, end, step;
+    template <class T>
+    __device__ __forceinline__ GroupLoop(const OpView<T> &op, int nb_plain, int per_block, int mine) {
+        const bool plain = (int)blockIdx.x < nb_plain;
+        const int64_t first = plain ? 0 : op.n_grp_plain, b = plain ? blockIdx.x : blockIdx.x - nb_plain;
+        g = first + b * per_block + mine;
+        end = plain ? op.n_grp_plain : op.n_grp;
+        step = per_block * (int64_t)(plain ? nb_plain : gridDim.x - nb_plain);
     }
+};
+
+// identity rows of a 32-slot pass, copied warp per row
+template <class T>
+__device__ __forceinline__ void e_ident32(const OpView<T> &op, int warp, int lane, bool act, const T *__restrict__ x,
+                                          T *__restrict__ t) {
     if (act)
         for (int64_t q = (int64_t)blockIdx.x * 4 + warp; q < op.n_ident; q += (int64_t)gridDim.x * 4) {
             const uint32_t r = (uint32_t)op.ident[q];
@@ -326,70 +328,14 @@ __global__ void __launch_bounds__(128) k_epass32s(OpView<T> op, const Slot *__re
         }
 }
 
-// IBC patch of one row of a 32-slot E pass (warp per row, lane = slot): patch-
-// list row q's value from its bulk value acc, sign (acc + sum_e w_e (x[new_e] -
-// x[old_e])) + xval x[xcol]: moved stencil points read the IBC DOF column
-// instead of the tube node (IBCMatrixManipulations::AddIBCExtension's column
-// moves, src/IBCMatrixManipulations.cpp:118-186); a point that moves to
-// several IBCs adds w x[target] for each further IBC (OpView::ov_*).  The lanes load 32 entries at
-// once and broadcast them, so a row's x loads are all in flight together.
-// q is the same in every lane; inactive slots (act false) load nothing.
-template <class T>
-__device__ __forceinline__ T ovl_e_patch(const int32_t *patch, const int32_t *ov_ptr, const int32_t *ov_col, const T *ov_w,
-                                         uint32_t r, T acc, int lane, bool act, const T *__restrict__ x) {
-    const int pi = patch[r];
-    for (int e = ov_ptr[2 * pi]; e < ov_ptr[2 * pi + 1]; ++e)
-        acc = fma_rn(ov_w[e], act ? x[(uint32_t)ov_col[e] * 32u + lane] : T(0), acc);
-    return acc;
-}
-
-template <class T, bool OVL>
-__device__ __forceinline__ T patch_row(const OpView<T> &op, int q, uint32_t r, T acc, int lane, bool act,
-                                       const T *__restrict__ x) {
-    const int e0 = op.pl_off[q], e1 = op.pl_off[q + 1], xc = op.pl_xcol[q], neg = op.pl_neg[q];
-    const T xv = op.pl_xval[q];
-    const T xe = (act && xc >= 0) ? x[(uint32_t)xc * 32u + lane] : T(0);
-    for (int base = e0; base < e1; base += 32) {
-        const int cnt = min(32, e1 - base);
-        int nc = 0, oc = 0;
-        T w = 0;
-        if (lane < cnt) {
-            nc = op.pe_new[base + lane];
-            oc = op.pe_old[base + lane];
-            w = op.pe_w[base + lane];
-        }
-        for (int u0 = 0; u0 < cnt; u0 += 8) {
-            T xn[8], xo[8], ww[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int k = u0 + u;
-                const uint32_t ncu = (uint32_t)__shfl_sync(FULL, nc, k & 31), ocu = (uint32_t)__shfl_sync(FULL, oc, k & 31);
-                ww[u] = __shfl_sync(FULL, w, k & 31);
-                const bool ok = act && k < cnt;
-                xn[u] = ok ? x[ncu * 32u + lane] : T(0);
-                xo[u] = ok ? x[ocu * 32u + lane] : T(0);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (u0 + u < cnt) acc = fma_rn(ww[u], sub_rn(xn[u], xo[u]), acc);
-        }
-    }
-    if constexpr (OVL)
-        if (neg & 2) acc = ovl_e_patch<T>(op.patch, op.ov_ptr, op.ov_col, op.ov_w, r, acc, lane, act, x);
-    if (neg & 1) acc = -acc;
-    if (xc >= 0) acc = fma_rn(xv, xe, acc);
-    return acc;
-}
-
-// 32 FP32 slots, warp per base group: the warp gathers the group's 64 x
-// values plane by plane (16 columns each) and keeps each pair of rows' sum in
-// registers (f32x2): plane i adds wx_i (sum_j wy_j sum_k wz_k x_ijk) in the
-// plane order of k_epass32s's combine, so the results are the same bit for
-// bit, with no block-level synchronisation and no shared partial sums.  Rows
-// EW_ROWS at a time; weights staged pair-interleaved in the warp's shared
-// memory.  Identity rows copied warp per row.  ph < 0: every slot.
+// 32 FP32 slots, warp per group: the warp gathers the group's 64 x values plane
+// by plane (16 columns each) and keeps each pair of rows' sum in registers
+// (f32x2): plane i adds wx_i (sum_j wy_j sum_k wz_k x_ijk) in plane order, with
+// no block-level synchronisation and no shared partial sums.  Rows EW_ROWS at a
+// time; weights staged pair-interleaved in the warp's shared memory.  Identity
+// rows copied warp per row.  ph < 0: every slot.
 constexpr int EW_ROWS = 8;
-__global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *__restrict__ sl, int ph,
+__global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *__restrict__ sl, int ph, int nb_plain,
                                                   const float *__restrict__ x, float *__restrict__ t) {
     __shared__ __align__(16) float sw[4][EW_ROWS * 12];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -397,8 +343,8 @@ __global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *
     if (!__any_sync(FULL, act)) return;  // the same 32 slots in every warp: block-uniform
     float *w = sw[warp];
     const float *__restrict__ xl = x + lane;
-    const int64_t W = (int64_t)gridDim.x * 4;
-    for (int64_t g = (int64_t)blockIdx.x * 4 + warp; g < op.n_grp; g += W) {
+    for (GroupLoop gl(op, nb_plain, 4, warp); gl.g < gl.end; gl.g += gl.step) {
+        const int64_t g = gl.g;
         const int p0 = op.grp[g], p1 = op.grp[g + 1];
         for (int c0 = p0; c0 < p1; c0 += EW_ROWS) {
             // rows in pairs, the odd row of a last pair with zero weights
@@ -409,7 +355,8 @@ __global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *
                 w[24 * (q >> 1) + 2 * c + (q & 1)] = q < nr ? op.w_ord[12 * (size_t)(c0 + q) + c] : 0.f;
             }
             const int row = lane < nr ? op.ord[c0 + lane] : 0;  // lane q: row q of the chunk
-            __syncwarp();
+            const int fl = lane < nr ? op.fl_ord[c0 + lane] & F_TERMS : 0;
+            const bool terms = __any_sync(FULL, fl != 0);
             uint64_t acc[EW_ROWS / 2];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -450,6 +397,11 @@ __global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *
                     float lo, hi;
                     f2_unpack(acc[p], lo, hi);
                     const int r0 = __shfl_sync(FULL, row, 2 * p), r1 = __shfl_sync(FULL, row, 2 * p + 1);
+                    if (terms) {
+                        const int f0 = __shfl_sync(FULL, fl, 2 * p), f1 = __shfl_sync(FULL, fl, 2 * p + 1);
+                        if (f0) lo = e_row_terms<float, 32>(op, (uint8_t)f0, r0, lane, lo, x);
+                        if (f1) hi = e_row_terms<float, 32>(op, (uint8_t)f1, r1, lane, hi, x);
+                    }
                     if (act) {
                         t[(uint32_t)r0 * 32u + lane] = lo;
                         if (2 * p + 1 < nr) t[(uint32_t)r1 * 32u + lane] = hi;
@@ -457,46 +409,260 @@ __global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *
                 }
         }
     }
-    if (act)
-        for (int64_t q = (int64_t)blockIdx.x * 4 + warp; q < op.n_ident; q += W) {
-            const uint32_t r = (uint32_t)op.ident[q];
-            t[r * 32u + lane] = x[r * 32u + lane];
-        }
+    e_ident32(op, warp, lane, act, x, t);
 }
 
-// 1 slot: one thread per row, rows visited in base-point order so that the
-// threads of a warp that share a base read the same cache lines.
+// a row that fixed point cannot hold, slot s of a K-wide batch
+template <int K>
+__device__ __noinline__ double e_row_fp64(const double *__restrict__ w, const int32_t *__restrict__ gc, int s,
+                                          const double *__restrict__ x) {
+    double acc = 0.0;
+    for (int i = 0; i < 4; ++i) {
+        double ay = 0.0;
+        for (int j = 0; j < 4; ++j) {
+            double az = 0.0;
+            for (int k = 0; k < 4; ++k) az += w[8 + k] * x[(int64_t)gc[16 * i + 4 * j + k] * K + s];
+            ay += w[4 + j] * az;
+        }
+        acc += w[i] * ay;
+    }
+    return acc;
+}
+
+__device__ __forceinline__ uint32_t exp_field(double v) { return (uint32_t)__double2hiint(v) & FX_EXP; }
+__device__ __forceinline__ bool nonzero(double v) { return ((uint32_t)__double2hiint(v) << 1 | (uint32_t)__double2loint(v)) != 0; }
+__device__ __forceinline__ Fx fx_from_double(double v, uint32_t e20) {
+    return fx_from_double((uint32_t)__double2hiint(v), (uint32_t)__double2loint(v), e20);
+}
+// nothing to align to (zeros, subnormals and values below 2^-895), or infinities and NaN
+__device__ __forceinline__ bool fx_out(uint32_t e20) { return e20 - FX_EMIN >= FX_EXP - FX_EMIN; }
+
+// 32 FP64 slots in fixed point (fixed62.h), two warps per group with 16 slots
+// each: lane (h, s) holds planes 2 h and 2 h + 1 of slot s, 32 values that are
+// aligned once and stay in registers for all rows of the group, and the two
+// halves of a slot add up by a shuffle.  (One warp with a whole stencil a lane
+// needs 255 registers; at eight warps an SM the multiply-add chains were exposed
+// and the pass took 435 us on the two-circle sphere at dx 0.025.)  The rows'
+// weights are broadcast from shared memory.
+constexpr int EX_ROWS = 8;
+__global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Slot *__restrict__ sl, int ph, int nb_plain,
+                                                     const double *__restrict__ x, double *__restrict__ t) {
+    __shared__ __align__(16) int2 sw[4][EX_ROWS * 12];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane >> 4, s = (lane & 15) + 16 * (warp & 1);
+    const bool act32 = (ph < 0) || sl[lane].phase == ph;
+    if (!__any_sync(FULL, act32)) return;  // the same 32 slots in every warp: block-uniform
+    const bool act = (ph < 0) || sl[s].phase == ph;
+    const double *__restrict__ xs = x + s;
+    const int2 *w0 = sw[warp];
+    GroupLoop gl(op, nb_plain, 2, warp >> 1);
+    if (!__any_sync(FULL, act)) gl.g = gl.end;
+    for (; gl.g < gl.end; gl.g += gl.step) {
+        const int64_t g = gl.g;
+        const int p0 = op.grp[g], p1 = op.grp[g + 1];
+        Fx v[32];
+        uint32_t e20 = 0;
+        {
+            double xv[32];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                int col[16];
+                e_group_cols(op.gcols, g, 2 * h + a, col);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) xv[16 * a + q] = act ? xs[(uint32_t)col[q] * 32u] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 32; ++q) e20 = max(e20, exp_field(xv[q]));
+            e20 = max(e20, __shfl_xor_sync(FULL, e20, 16));
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] = fx_from_double(xv[q], e20);
+        }
+        const bool out = act && fx_out(e20), any_out = __any_sync(FULL, out);
+        for (int c0 = p0; c0 < p1; c0 += EX_ROWS) {
+            const int nr = min(p1 - c0, EX_ROWS);
+            __syncwarp();
+            for (int e = lane; e < 6 * nr; e += 32) ((int4 *)sw[warp])[e] = __ldg((const int4 *)(op.w_fix + 12 * (size_t)c0) + e);
+            const int row = lane < nr ? op.ord[c0 + lane] : 0;  // lane q: row q of the chunk
+            const int fl = lane < nr ? op.fl_ord[c0 + lane] & F_TERMS : 0;
+            __syncwarp();
+            for (int q = 0; q < nr; ++q) {
+                const int2 *w = w0 + 12 * q;
+                Fx wy[4], wz[4];
+                fx_lds4(w + 4, wy);
+                fx_lds4(w + 8, wz);
+                FxSum sum;
+                if (h) sum.c = 0;  // the rounding bit once
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    Fx ay[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const Fx *l = v + 16 * a + 4 * j;
+                        const Fx line[4] = {l[0], l[1], l[2], l[3]};
+                        ay[j] = fx_split(fx_dot4(line, wz));
+                    }
+                    sum.add(fx_split(fx_dot4(ay, wy)), fx_lds1(w + 2 * h + a));
+                }
+                sum.c += __shfl_xor_sync(FULL, sum.c, 16);
+                sum.a += __shfl_xor_sync(FULL, sum.a, 16);
+                const int r = __shfl_sync(FULL, row, q), f = __shfl_sync(FULL, fl, q);
+                if (h == 0 && act && !out) {
+                    double acc = fx_to_double(sum.get(), e20);
+                    if (f) acc = e_row_terms<double, 32>(op, (uint8_t)f, r, s, acc, x);
+                    t[(uint32_t)r * 32u + s] = acc;
+                }
+            }
+        }
+        if (any_out) {  // these slots again, in FP64 (zeros stay zeros)
+            bool nz = false;
+            if (out)
+                for (int q = 0; q < 64; ++q) nz = nz || nonzero(xs[(uint32_t)op.gcols[64 * g + q] * 32u]);
+            for (int p = p0; p < p1; ++p)
+                if (out && h == 0) {
+                    const int r = op.ord[p], f = op.fl_ord[p] & F_TERMS;
+                    double acc = nz ? e_row_fp64<32>(op.w_ord + 12 * (size_t)p, op.gcols + 64 * g, s, x) : 0.0;
+                    if (f) acc = e_row_terms<double, 32>(op, (uint8_t)f, r, s, acc, x);
+                    t[(uint32_t)r * 32u + s] = acc;
+                }
+        }
+    }
+    e_ident32(op, warp, lane, act32, x, t);
+}
+
+// 1 slot: a warp per run of at most 32 rows of at most E1_GROUPS groups, a lane
+// per row.  The warp gathers each group's 64 values together (two a lane, in the
+// group table's order, so neighbouring lanes mostly read one line, and the
+// gathers of all groups are in flight at once) and leaves them in shared memory,
+// where each row reads its group's.  FP64 values are aligned to their group's
+// exponent on the way and summed in fixed point (fixed62.h).
+constexpr int E1_T = 128;
+
+// the 64 values of a group in shared memory; the pad keeps different groups' reads on different banks
 template <class T>
-__global__ void k_epass1(OpView<T> op, const Slot *__restrict__ sl, int ph, const T *__restrict__ x, T *__restrict__ t) {
+struct E1Group;
+template <>
+struct E1Group<float> {
+    alignas(16) float x[68];
+};
+template <>
+struct E1Group<double> {
+    alignas(16) Fx x[66];
+};
+
+__device__ __forceinline__ float e1_row(const OpView<float> &op, int64_t p, uint32_t, const E1Group<float> &g) {
+    float w[12];
+    load_w12(op.w_ord + 12 * p, w);
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float ay = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float v[4];
+            lds4(g.x + 16 * i + 4 * j, v);
+            float az = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) az += w[8 + k] * v[k];
+            ay += w[4 + j] * az;
+        }
+        acc += w[i] * ay;
+    }
+    return acc;
+}
+
+__device__ __forceinline__ double e1_row(const OpView<double> &op, int64_t p, uint32_t e20, const E1Group<double> &g) {
+    const int2 *w = op.w_fix + 12 * p;
+    Fx wx[4], wy[4], wz[4], ax[4];
+    fx_load4(w, wx);
+    fx_load4(w + 4, wy);
+    fx_load4(w + 8, wz);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        Fx ay[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int4 *l = (const int4 *)(g.x + 16 * i + 4 * j);
+            const int4 a = l[0], b = l[1];
+            const Fx v[4] = {Fx{a.x, a.y}, Fx{a.z, a.w}, Fx{b.x, b.y}, Fx{b.z, b.w}};
+            ay[j] = fx_split(fx_dot4(v, wz));
+        }
+        ax[i] = fx_split(fx_dot4(ay, wy));
+    }
+    return fx_to_double(fx_dot4(ax, wx), e20);
+}
+
+template <class T>
+__global__ void __launch_bounds__(E1_T) k_epass1(OpView<T> op, const Slot *__restrict__ sl, int ph, unsigned row_blocks,
+                                                 const T *__restrict__ x, T *__restrict__ t) {
+    __shared__ E1Group<T> sh[E1_T / 32][E1_GROUPS];
     if (ph >= 0 && sl[0].phase != ph) return;
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p < op.n_ord) {
-        const int64_t r = op.ord[p];
-        t[r] = e_row_thread<T, 1>(op, r, 0, x);
+    if (blockIdx.x >= row_blocks) {  // identity rows
+        const int64_t q = (int64_t)(blockIdx.x - row_blocks) * E1_T + threadIdx.x;
+        if (q < op.n_ident) {
+            const int r = op.ident[q];
+            t[r] = x[r];
+        }
         return;
     }
-    const int64_t q = p - op.n_ord;
-    if (q < op.n_ident) {
-        const int64_t r = op.ident[q];
-        t[r] = x[r];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * (E1_T / 32) + warp;
+    if (c >= op.n_chunk) return;
+    const int4 ch = __ldg(op.chunk + c);
+    const int ng = ch.w >> 8, nr = ch.w & 255;
+    const int32_t *gc = op.gcols + 64 * (int64_t)ch.x + lane;
+    T xa[E1_GROUPS], xb[E1_GROUPS];
+    {
+        int ca[E1_GROUPS], cb[E1_GROUPS];
+#pragma unroll
+        for (int g = 0; g < E1_GROUPS; ++g)
+            if (g < ng) {
+                ca[g] = __ldg(gc + 64 * g);
+                cb[g] = __ldg(gc + 64 * g + 32);
+            }
+#pragma unroll
+        for (int g = 0; g < E1_GROUPS; ++g)
+            if (g < ng) {
+                xa[g] = x[ca[g]];
+                xb[g] = x[cb[g]];
+            }
     }
-}
-
-// the patch as a pass of its own after the bulk 32-slot E pass, warp per
-// patch-list row (consecutive rows on neighbouring warps, whose gathers share
-// cache lines)
-template <class T, bool OVL>
-__global__ void __launch_bounds__(128) k_epatch32(OpView<T> op, const Slot *__restrict__ sl, int ph, const T *__restrict__ x,
-                                                  T *__restrict__ t) {
-    const int lane = threadIdx.x & 31;
-    const bool act = (ph < 0) || sl[lane].phase == ph;
-    if (!__any_sync(FULL, act)) return;  // the same slots in every warp: block-uniform
-    const int64_t warps = (int64_t)gridDim.x * 4;
-    for (int64_t q = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5); q < op.n_pl; q += warps) {
-        const uint32_t r = (uint32_t)op.pl_row[q];
-        const T acc = act ? t[r * 32u + lane] : T(0);
-        const T v = patch_row<T, OVL>(op, (int)q, r, acc, lane, act, x);
-        if (act) t[r * 32u + lane] = v;
+    const int64_t p = ch.y + min(lane, nr - 1);
+    const int mine = __popc((uint32_t)ch.z & (0xffffffffu >> (31 - lane))) - 1;  // the row's group
+    const int r = __ldg(op.ord + p);
+    const uint8_t fl = __ldg(op.fl_ord + p) & F_TERMS;
+    uint32_t e20 = FX_EMIN;  // exponent field of the row's group
+    bool zero = false;       // the warp's groups of smallest exponent hold zeros only
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+        for (int g = 0; g < E1_GROUPS; ++g)
+            if (g < ng) {
+                const uint32_t e = __reduce_max_sync(FULL, max(exp_field(xa[g]), exp_field(xb[g])));
+                if (mine == g) e20 = e;
+                sh[warp][g].x[lane] = fx_from_double(xa[g], e);
+                sh[warp][g].x[lane + 32] = fx_from_double(xb[g], e);
+            }
+        if (__any_sync(FULL, e20 == 0)) {
+            bool nz = false;
+#pragma unroll
+            for (int g = 0; g < E1_GROUPS; ++g)
+                if (g < ng) nz = nz || nonzero(xa[g]) || nonzero(xb[g]);
+            nz = __any_sync(FULL, nz);  // every lane votes
+            zero = e20 == 0 && !nz;
+        }
+    } else {
+#pragma unroll
+        for (int g = 0; g < E1_GROUPS; ++g)
+            if (g < ng) {
+                sh[warp][g].x[lane] = xa[g];
+                sh[warp][g].x[lane + 32] = xb[g];
+            }
+    }
+    __syncwarp();
+    T acc = e1_row(op, p, e20, sh[warp][mine]);
+    if constexpr (sizeof(T) == 8)
+        if (fx_out(e20)) acc = zero ? 0.0 : e_row_fp64<1>(op.w_ord + 12 * p, op.gcols + 64 * (int64_t)(ch.x + mine), 0, x);
+    if (lane < nr) {
+        if (fl) acc = e_row_terms<T, 1>(op, fl, r, 0, acc, x);
+        t[r] = acc;
     }
 }
 
@@ -532,42 +698,37 @@ static void slot_epatch(const OpView<T> &op, const Slot *sl, int ph, const T *x,
 }
 
 // default launch shapes of the 32-slot E passes (blocks per SM caps of the
-// grid-stride loops): the FP32 bulk pass's best on the sphere with two circles at
-// dx 0.025; for the patch and FP64 passes the autotuner chose 64 or more blocks
-// per SM on the sphere, the torus and the mesh of the serving stream
+// grid-stride loops over the groups without and with moved columns)
 constexpr int E32_BPS = 32, PATCH_BPS = 64, E64_BPS = 64;
 
 // kernels one E pass of x launches
 template <class T, int K>
 static inline int epass_kernels(const OpView<T> &op, const T *) {
-    const int sp = (K == 32 && op.n_sp_rows > 0) ? 1 : 0;
-    return ((K == 32 && op.n_pl > 0) ? 2 : 1) + sp;
+    return (K == 32 && op.n_sp_rows > 0) ? 2 : 1;
+}
+
+// blocks of a 32-slot pass over n groups: four a block (FP32) or two (FP64)
+template <class T>
+static inline int group_blocks(int64_t n, int bps) {
+    constexpr int per = sizeof(T) == 4 ? 4 : 2;
+    return (int)std::min<int64_t>((n + per - 1) / per, (int64_t)bps * sm_count());
 }
 
 template <class T, int K>
 static void launch_epass(const OpView<T> &op, const Slot *sl, int ph, const T *x, T *t, cudaStream_t st) {
     static_assert(K == 1 || K == 32, "slot widths 1 and 32");
     if constexpr (K == 32) {
-        if constexpr (sizeof(T) == 4) {
-            const int64_t bps = op.e32_bps > 0 ? op.e32_bps : E32_BPS;
-            const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((op.n_grp + 3) / 4, bps * sm_count()));
-            k_epass32w<<<(unsigned)blocks, 128, 0, st>>>(op, sl, ph, x, t);
-        } else {
-            const int64_t bps = op.e64_bps > 0 ? op.e64_bps : E64_BPS;
-            const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(op.n_grp, bps * sm_count()));
-            k_epass32s<T><<<(unsigned)blocks, 128, 0, st>>>(op, sl, ph, x, t);
-        }
-    } else {
-        const int64_t threads = op.n_ord + op.n_ident;
-        k_epass1<T><<<(unsigned)((threads + BS - 1) / BS), BS, 0, st>>>(op, sl, ph, x, t);
-    }
-    if (K == 32 && op.n_pl > 0) {  // the gather passes correct the IBC patch rows afterwards
-        const int64_t bps = op.patch_bps > 0 ? op.patch_bps : PATCH_BPS;
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((op.n_pl + 3) / 4, bps * sm_count()));
-        if (op.ov_ptr)
-            k_epatch32<T, true><<<(unsigned)blocks, 128, 0, st>>>(op, sl, ph, x, t);
+        const int bps = sizeof(T) == 4 ? (op.e32_bps > 0 ? op.e32_bps : E32_BPS) : (op.e64_bps > 0 ? op.e64_bps : E64_BPS);
+        const int plain = group_blocks<T>(op.n_grp_plain, bps);
+        const int crossing = group_blocks<T>(op.n_grp - op.n_grp_plain, op.patch_bps > 0 ? op.patch_bps : PATCH_BPS);
+        const unsigned blocks = (unsigned)std::max(1, plain + crossing);
+        if constexpr (sizeof(T) == 4)
+            k_epass32w<<<blocks, 128, 0, st>>>(op, sl, ph, plain, x, t);
         else
-            k_epatch32<T, false><<<(unsigned)blocks, 128, 0, st>>>(op, sl, ph, x, t);
+            k_epass32x<<<blocks, 128, 0, st>>>(op, sl, ph, plain, x, t);
+    } else {
+        const unsigned rows = (unsigned)((op.n_chunk + E1_T / 32 - 1) / (E1_T / 32)), id = (unsigned)((op.n_ident + E1_T - 1) / E1_T);
+        k_epass1<T><<<std::max(1u, rows + id), E1_T, 0, st>>>(op, sl, ph, rows, x, t);
     }
     if (K == 32 && op.n_sp_rows > 0) slot_epatch(op, sl, ph, x, t, st);
 }
@@ -2449,26 +2610,23 @@ extern "C" int cpm_opset_autotune(cpm_opset_t op, int32_t reps, int32_t with_fp6
             best_us = dflt_us;
         }
     };
-    if (op->n_grp > 0) {
+    // one range of groups alone: the others get no block
+    if (v32.n_grp_plain > 0) {
         pick(e32c, 8, E32_BPS, [&](int bps) {
-            const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((v32.n_grp + 3) / 4, (int64_t)bps * sms));
-            k_epass32w<<<(unsigned)blocks, 128, 0, st>>>(v32, nullptr, -1, x32.p, t32.p);
+            const int blocks = group_blocks<float>(v32.n_grp_plain, bps);
+            k_epass32w<<<blocks, 128, 0, st>>>(v32, nullptr, -1, blocks, x32.p, t32.p);
         }, res.e32_us, res.e32_default_us, res.e32_blocks_per_sm);
     }
-    if (op->n_pl > 0) {
+    if (v32.n_grp > v32.n_grp_plain) {
         pick(pc, 6, PATCH_BPS, [&](int bps) {
-            const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((v32.n_pl + 3) / 4, (int64_t)bps * sms));
-            if (v32.ov_ptr)
-                k_epatch32<float, true><<<(unsigned)blocks, 128, 0, st>>>(v32, nullptr, -1, x32.p, t32.p);
-            else
-                k_epatch32<float, false><<<(unsigned)blocks, 128, 0, st>>>(v32, nullptr, -1, x32.p, t32.p);
+            k_epass32w<<<group_blocks<float>(v32.n_grp - v32.n_grp_plain, bps), 128, 0, st>>>(v32, nullptr, -1, 0, x32.p, t32.p);
         }, res.patch_us, res.patch_default_us, res.patch_blocks_per_sm);
     }
-    if (with_fp64 && op->n_grp > 0) {
+    if (with_fp64 && op->n_grp_plain > 0) {
         const OpView<double> v64 = op->view<double>();
         pick(e64c, 5, E64_BPS, [&](int bps) {
-            const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(v64.n_grp, (int64_t)bps * sms));
-            k_epass32s<double><<<(unsigned)blocks, 128, 0, st>>>(v64, nullptr, -1, x64.p, t64.p);
+            const int blocks = group_blocks<double>(v64.n_grp_plain, bps);
+            k_epass32x<<<blocks, 128, 0, st>>>(v64, nullptr, -1, blocks, x64.p, t64.p);
         }, res.e64_us, res.e64_default_us, res.e64_blocks_per_sm);
     }
     CPM_CUDA_TRY(cudaGetLastError());

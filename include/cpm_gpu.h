@@ -263,8 +263,9 @@ int cpm_apply_device(cpm_opset_t op, double m, double n, int32_t kslots, int32_t
                      void *y_dev);
 
 /* Launch shapes of an operator's 32-slot E passes, as blocks per SM of their
- * grid-stride loops: the FP32 bulk pass, the IBC patch pass and the FP64 bulk
- * pass (0 keeps the built-in default).  They never change results.  No
+ * grid-stride loops: the FP32 pass over the rows without moved columns, either
+ * pass over the rows whose stencil crosses an IBC ("patch"), and the FP64 pass
+ * over the rows without (0 keeps the built-in default).  They never change results.  No
  * counterpart in the reference, whose E is a CPU sparse product. */
 typedef struct {
     int32_t e32_blocks_per_sm, patch_blocks_per_sm, e64_blocks_per_sm;
