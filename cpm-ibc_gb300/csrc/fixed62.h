@@ -51,6 +51,17 @@ __device__ __forceinline__ Fx fx_from_double(uint32_t hi, uint32_t lo, uint32_t 
     return fx_split((int64_t)((((uint64_t)((uint32_t)(v >> 32) ^ s)) << 32) | (uint64_t)((uint32_t)v ^ s)));
 }
 
+// the double v in units of 2^(e - 59), 60 bits: six of them add up without overflow
+__device__ __forceinline__ int64_t fx60_from_double(double v, uint32_t e20) {
+    const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+    const uint32_t d = min((e20 - (hi & FX_EXP)) >> 20, 63u);
+    const uint32_t mh = (hi & 0xfffffu) | 0x100000u;
+    const uint64_t m = ((uint64_t)__funnelshift_l(lo, mh, 7) << 32) | (uint64_t)(lo << 7);
+    const uint64_t r = m >> d;
+    const uint32_t s = (uint32_t)((int)hi >> 31);
+    return (int64_t)((((uint64_t)((uint32_t)(r >> 32) ^ s)) << 32) | (uint64_t)((uint32_t)r ^ s));
+}
+
 // a b + c on 32-bit signed factors
 __device__ __forceinline__ int64_t fx_mad(int a, int b, int64_t c) {
     int64_t d;

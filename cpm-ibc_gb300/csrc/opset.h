@@ -375,6 +375,36 @@ __device__ __forceinline__ T ovl_l_term(const OpView<T> &op, int64_t r, int s, T
     return n * (op.Loff * a);
 }
 
+// The FP64 seven-point row c0 x + c1 sum_d t_d of at most six neighbours (0 where
+// absent).  Six FP64 additions and the products were the L pass's bound (81 % of
+// the FP64 pipe, 145 us for 32 slots on the two-circle sphere at dx 0.025), so
+// the sum runs in fixed point aligned to the largest neighbour: exact but for the
+// last of 60 bits, rounded once to FP64.  The power of two goes into c1's
+// exponent; values or a c1 near the ends of the exponent range take the FP64 sum.
+struct LCoef {
+    double c0, c1;
+    bool c1_mid;  // |c1| within 2^-64 .. 2^64
+    __device__ __forceinline__ LCoef(double m, double n, double Ldiag, double Loff)
+        : c0(fma(n, Ldiag, m)), c1(n * Loff), c1_mid(fabs(c1) >= 0x1p-64 && fabs(c1) <= 0x1p64) {}
+};
+__device__ __forceinline__ double l_row(const LCoef &lc, double x, const double (&t)[6]) {
+    uint32_t e20 = 0;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) e20 = max(e20, (uint32_t)__double2hiint(t[d]) & FX_EXP);
+    const double cx = lc.c0 * x;
+    if (!lc.c1_mid || e20 - (200u << 20) >= (1700u << 20)) {
+        double off = 0.0;
+#pragma unroll
+        for (int d = 0; d < 6; ++d) off += t[d];
+        return fma(lc.c1, off, cx);
+    }
+    int64_t v = 0;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) v += fx60_from_double(t[d], e20);
+    const double c1 = __hiloint2double(__double2hiint(lc.c1) + (int)(e20 - (1082u << 20)), __double2loint(lc.c1));
+    return fma(c1, (double)v, cx);
+}
+
 // y_r = m x_r + n (Ldiag x_r + Loff sum_d t_{c_d}), identity rows y = x
 // (GeneralizedBiCGStabSystem::Multiply, src/GeneralizedBiCGStabSystem.h:191-233)
 // for slot s of a K-wide row-major batch and U rows at once: the flags, x and
@@ -405,16 +435,16 @@ __device__ __forceinline__ void l_rows(const OpView<T> &op, const int64_t (&r)[U
         c[u][4] = e.x;
         c[u][5] = e.y;
     }
+    T tv[U][6];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int d = 0; d < 6; ++d)
+            tv[u][d] = (c[u][d] >= 0 && act && !(fl[u] & F_IDENT)) ? t[(int64_t)c[u][d] * K + s] : T(0);
     if constexpr (sizeof(T) == 8) {
+        const LCoef lc(m, n, op.Ldiag, op.Loff);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            T off = 0;
-#pragma unroll
-            for (int d = 0; d < 6; ++d)
-                if (c[u][d] >= 0 && act && !(fl[u] & F_IDENT)) off += t[(int64_t)c[u][d] * K + s];
-            y[u] = (fl[u] & F_IDENT) ? xr[u] : m * xr[u] + n * (op.Ldiag * xr[u] + op.Loff * off);
-            if ((fl[u] & F_SLOTP) && act) y[u] += slot_l_correction<T, K>(op, r[u], s, n, t);
-        }
+        for (int u = 0; u < U; ++u) y[u] = (fl[u] & F_IDENT) ? xr[u] : l_row(lc, xr[u], tv[u]);
     } else {
         // FP32: the same row as Loff (sum_d (t_d - x) + (k - 6) x) with k present
         // neighbours (Ldiag = -6 Loff).  The differences of a smooth field are
@@ -426,17 +456,18 @@ __device__ __forceinline__ void l_rows(const OpView<T> &op, const int64_t (&r)[U
 #pragma unroll
             for (int d = 0; d < 6; ++d)
                 if (c[u][d] >= 0 && act && !(fl[u] & F_IDENT)) {
-                    off += t[(int64_t)c[u][d] * K + s] - xr[u];
+                    off += tv[u][d] - xr[u];
                     ++k;
                 }
             off += (T)(k - 6) * xr[u];
             y[u] = (fl[u] & F_IDENT) ? xr[u] : m * xr[u] + n * (op.Loff * off);
-            if ((fl[u] & F_SLOTP) && act) y[u] += slot_l_correction<T, K>(op, r[u], s, n, t);
         }
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+    for (int u = 0; u < U; ++u) {
+        if ((fl[u] & F_SLOTP) && act) y[u] += slot_l_correction<T, K>(op, r[u], s, n, t);
         if ((fl[u] & F_OVL) && act) y[u] += ovl_l_term<T, K>(op, r[u], s, n, t);
+    }
 }
 
 // l_rows for 32 FP32 slots, four per thread: slots 4q .. 4q+3 of U rows, as

@@ -70,8 +70,10 @@ constexpr int UNR = 4;       // rows in flight per thread in the row loops
 constexpr int RGROUP = 32;   // blocks per first-level group of the grid reduction
 constexpr unsigned FULL = 0xffffffffu;
 
-// grid size of the row-loop kernels: UNR rows per thread per trip, at most
-// four 256-thread blocks per SM (the reduction tree is fixed by this size)
+// grid size of the row-loop kernels: at most four 256-thread blocks per SM, and
+// one row per thread until these are reached (with four rows a thread, 22
+// thousand rows kept 23 of 152 SMs busy: 8.9 us for one L pass).  The reduction
+// tree is fixed by this size.
 static inline int sm_count() {
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
@@ -81,7 +83,7 @@ static inline int sm_count() {
 static inline int row_grid(int64_t D, int K) {
     const int sms = sm_count();
     const int64_t rpb = BS / K;
-    const int64_t need = (D + rpb * UNR - 1) / (rpb * UNR);
+    const int64_t need = (D + rpb - 1) / rpb;
     return (int)std::max<int64_t>(1, std::min<int64_t>(need, 4LL * sms));
 }
 static inline int64_t reduce_groups(int G) { return (G + RGROUP - 1) / RGROUP; }
@@ -758,7 +760,7 @@ int epass64_batch(const cpm_opset_s *o, bool slot_patches, const double *x, doub
     _Pragma("unroll") for (int u = 0; u < (UN); ++u) rr[u] = rb + (int64_t)u * rstride;
 #define ROWS_UNR(Dn) ROWS_UNR_N(Dn, UNR)
 #define ROWS_OF_TRIP(rr) ROWS_OF_TRIP_N(rr, UNR)
-// FP64 streams of six vectors keep two rows in flight within 64 registers
+// FP64 streams of six vectors and FP64 L rows keep two rows in flight within 64 registers
 template <class T>
 constexpr int unr_stream6() { return sizeof(T) == 8 ? 2 : UNR; }
 
@@ -767,12 +769,13 @@ template <class T, int K>
 __global__ void __launch_bounds__(BS, 4) k_lpass(OpView<T> op, T m, T n, const T *__restrict__ x, const T *__restrict__ t,
                                               T *__restrict__ y) {
     GRID_LOOP
-    ROWS_UNR(op.D) {
-        ROWS_OF_TRIP(rr)
-        T v[UNR];
-        l_rows<T, K, UNR>(op, rr, s, m, n, x, t, true, v);
+    constexpr int UN = unr_stream6<T>();
+    ROWS_UNR_N(op.D, UN) {
+        ROWS_OF_TRIP_N(rr, UN)
+        T v[UN];
+        l_rows<T, K, UN>(op, rr, s, m, n, x, t, true, v);
 #pragma unroll
-        for (int u = 0; u < UNR; ++u)
+        for (int u = 0; u < UN; ++u)
             if (rr[u] < op.D) y[rr[u] * K + s] = v[u];
     }
 }
@@ -853,11 +856,13 @@ __global__ void __launch_bounds__(BS, 4) k_init(OpView<T> op, Slot *sl, SolvePar
 }
 
 // p = (p - w v) beta + r ; y = M^-1 p   (src/BiCGStab.h:74-78)
-// M^-1 here is the diagonal inverse (ys = 1, pden = m + n L_rr), the identity
-// (pden = null) or the first Jacobi sweep from zero, y = omega (p / pden)
+// M^-1 here is the diagonal inverse (ys = 1, pinv = 1 / (m + n L_rr)), the identity
+// (pinv = null) or the first Jacobi sweep from zero, y = omega (p pinv).  The
+// quotient itself was ten of the thirteen FP64 operations of a row here; the
+// rounding of M^-1 does not enter x, which is updated by the y that A was applied to.
 // (src/GeneralizedBiCGStabSystem.h:358-377 with result = 0 and A 0 = 0)
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_update_p(int64_t D, const Slot *__restrict__ sl, const T *__restrict__ pden, T ys,
+__global__ void __launch_bounds__(BS, 4) k_update_p(int64_t D, const Slot *__restrict__ sl, const T *__restrict__ pinv, T ys,
                                                  const T *__restrict__ r, const T *__restrict__ v, T *__restrict__ p,
                                                  T *__restrict__ y, T *__restrict__ r0) {
     GRID_LOOP
@@ -875,7 +880,7 @@ __global__ void __launch_bounds__(BS, 4) k_update_p(int64_t D, const Slot *__res
                 pv[u] = p[i];
                 vv[u] = v[i];
                 rv[u] = r[i];
-                dv[u] = pden ? pden[rr[u]] : T(1);
+                dv[u] = pinv ? pinv[rr[u]] : T(1);
             }
 #pragma unroll
         for (int u = 0; u < UN; ++u)
@@ -889,7 +894,7 @@ __global__ void __launch_bounds__(BS, 4) k_update_p(int64_t D, const Slot *__res
                     r0[i] = pi;
                 }
                 p[i] = pi;
-                y[i] = pden ? ys * (pi / dv[u]) : pi;
+                y[i] = pinv ? ys * (pi * dv[u]) : pi;
             }
     }
 }
@@ -900,17 +905,18 @@ __global__ void __launch_bounds__(BS, 4) k_apply_alpha(OpView<T> op, Slot *sl, T
                                                     const T *__restrict__ te, const T *__restrict__ r0, T *__restrict__ v,
                                                     double *partial, unsigned int *counter) {
     GRID_LOOP
+    constexpr int UN = unr_stream6<T>();
     const bool act = sl[s].phase == PH_ITER;
     Dot<T, 1> acc;
     if (act)
-        ROWS_UNR(op.D) {
-            ROWS_OF_TRIP(rr)
-            T r0v[UNR], vv[UNR];
+        ROWS_UNR_N(op.D, UN) {
+            ROWS_OF_TRIP_N(rr, UN)
+            T r0v[UN], vv[UN];
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) r0v[u] = rr[u] < op.D ? r0[rr[u] * K + s] : T(0);
-            l_rows<T, K, UNR>(op, rr, s, m, n, y, te, true, vv);
+            for (int u = 0; u < UN; ++u) r0v[u] = rr[u] < op.D ? r0[rr[u] * K + s] : T(0);
+            l_rows<T, K, UN>(op, rr, s, m, n, y, te, true, vv);
 #pragma unroll
-            for (int u = 0; u < UNR; ++u)
+            for (int u = 0; u < UN; ++u)
                 if (rr[u] < op.D) {
                     v[rr[u] * K + s] = vv[u];
                     acc.add(0, r0v[u], vv[u]);
@@ -923,7 +929,7 @@ __global__ void __launch_bounds__(BS, 4) k_apply_alpha(OpView<T> op, Slot *sl, T
 
 // s = r - alpha v ; z = M^-1 s   (src/BiCGStab.h:82-84), M^-1 as in k_update_p
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_update_s(int64_t D, const Slot *__restrict__ sl, const T *__restrict__ pden, T ys,
+__global__ void __launch_bounds__(BS, 4) k_update_s(int64_t D, const Slot *__restrict__ sl, const T *__restrict__ pinv, T ys,
                                                  const T *__restrict__ r, const T *__restrict__ v, T *__restrict__ sv,
                                                  T *__restrict__ z) {
     GRID_LOOP
@@ -938,7 +944,7 @@ __global__ void __launch_bounds__(BS, 4) k_update_s(int64_t D, const Slot *__res
                 const int64_t i = rr[u] * K + s;
                 vv[u] = v[i];
                 rv[u] = r[i];
-                dv[u] = pden ? pden[rr[u]] : T(1);
+                dv[u] = pinv ? pinv[rr[u]] : T(1);
             }
 #pragma unroll
         for (int u = 0; u < UNR; ++u)
@@ -946,35 +952,36 @@ __global__ void __launch_bounds__(BS, 4) k_update_s(int64_t D, const Slot *__res
                 const int64_t i = rr[u] * K + s;
                 T si = -a * vv[u] + rv[u];
                 sv[i] = si;
-                z[i] = pden ? ys * (si / dv[u]) : si;
+                z[i] = pinv ? ys * (si * dv[u]) : si;
             }
     }
 }
 
 // one further damped Jacobi sweep on A y = c, after the E pass te = E~ y:
-// y += omega ((c - A y) / pden)   (src/GeneralizedBiCGStabSystem.h:366-376).
+// y += omega ((c - A y) pinv)   (src/GeneralizedBiCGStabSystem.h:366-376).
 // Row r of A y reads y only at row r, so the update is in place.
 template <class T, int K>
 __global__ void __launch_bounds__(BS, 4) k_jacobi_sweep(OpView<T> op, const Slot *__restrict__ sl, T m, T n,
                                                      const T *__restrict__ c, const T *__restrict__ te,
-                                                     const T *__restrict__ pden, T omega, T *y) {
+                                                     const T *__restrict__ pinv, T omega, T *y) {
     GRID_LOOP
+    constexpr int UN = unr_stream6<T>();
     if (sl[s].phase != PH_ITER) return;
-    ROWS_UNR(op.D) {
-        ROWS_OF_TRIP(rr)
-        T cv[UNR], dv[UNR], ay[UNR];
+    ROWS_UNR_N(op.D, UN) {
+        ROWS_OF_TRIP_N(rr, UN)
+        T cv[UN], dv[UN], ay[UN];
 #pragma unroll
-        for (int u = 0; u < UNR; ++u)
+        for (int u = 0; u < UN; ++u)
             if (rr[u] < op.D) {
                 cv[u] = c[rr[u] * K + s];
-                dv[u] = pden[rr[u]];
+                dv[u] = pinv[rr[u]];
             }
-        l_rows<T, K, UNR>(op, rr, s, m, n, y, te, true, ay);
+        l_rows<T, K, UN>(op, rr, s, m, n, y, te, true, ay);
 #pragma unroll
-        for (int u = 0; u < UNR; ++u)
+        for (int u = 0; u < UN; ++u)
             if (rr[u] < op.D) {
                 const int64_t i = rr[u] * K + s;
-                y[i] = y[i] + omega * ((cv[u] - ay[u]) / dv[u]);
+                y[i] = y[i] + omega * ((cv[u] - ay[u]) * dv[u]);
             }
     }
 }
@@ -985,17 +992,18 @@ __global__ void __launch_bounds__(BS, 4) k_apply_omega(OpView<T> op, Slot *sl, T
                                                     const T *__restrict__ te, const T *__restrict__ sv, T *__restrict__ tv,
                                                     double *partial, unsigned int *counter) {
     GRID_LOOP
+    constexpr int UN = unr_stream6<T>();
     const bool act = sl[s].phase == PH_ITER;
     Dot<T, 2> acc;
     if (act)
-        ROWS_UNR(op.D) {
-            ROWS_OF_TRIP(rr)
-            T svv[UNR], tt[UNR];
+        ROWS_UNR_N(op.D, UN) {
+            ROWS_OF_TRIP_N(rr, UN)
+            T svv[UN], tt[UN];
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) svv[u] = rr[u] < op.D ? sv[rr[u] * K + s] : T(0);
-            l_rows<T, K, UNR>(op, rr, s, m, n, z, te, true, tt);
+            for (int u = 0; u < UN; ++u) svv[u] = rr[u] < op.D ? sv[rr[u] * K + s] : T(0);
+            l_rows<T, K, UN>(op, rr, s, m, n, z, te, true, tt);
 #pragma unroll
-            for (int u = 0; u < UNR; ++u)
+            for (int u = 0; u < UN; ++u)
                 if (rr[u] < op.D) {
                     tv[rr[u] * K + s] = tt[u];
                     acc.add(0, tt[u], tt[u]);
@@ -1316,18 +1324,19 @@ __global__ void __launch_bounds__(BS, 4) k_restart(OpView<T> op, Slot *sl, T m, 
                                                 const T *__restrict__ x, const T *__restrict__ te, T *__restrict__ r,
                                                 T *__restrict__ r0, double *partial, unsigned int *counter) {
     GRID_LOOP
+    constexpr int UN = unr_stream6<T>();
     const bool act = sl[s].phase == PH_RESTART;
     Dot<T, 1> acc;
     if (act)
-        ROWS_UNR(op.D) {
-            ROWS_OF_TRIP(rr)
-            double bv[UNR];
-            T ax[UNR];
+        ROWS_UNR_N(op.D, UN) {
+            ROWS_OF_TRIP_N(rr, UN)
+            double bv[UN];
+            T ax[UN];
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) bv[u] = rr[u] < op.D ? b[rr[u] * K + s] : 0.0;
-            l_rows<T, K, UNR>(op, rr, s, m, n, x, te, true, ax);
+            for (int u = 0; u < UN; ++u) bv[u] = rr[u] < op.D ? b[rr[u] * K + s] : 0.0;
+            l_rows<T, K, UN>(op, rr, s, m, n, x, te, true, ax);
 #pragma unroll
-            for (int u = 0; u < UNR; ++u)
+            for (int u = 0; u < UN; ++u)
                 if (rr[u] < op.D) {
                     const int64_t i = rr[u] * K + s;
                     T ri = (T)bv[u] - ax[u];
@@ -1380,17 +1389,18 @@ __global__ void __launch_bounds__(BS, 4) k_refine_residual(OpView<double> op, Sl
                                                         const double *__restrict__ te, double *__restrict__ r64,
                                                         double *partial, unsigned int *counter) {
     GRID_LOOP
+    constexpr int UN = unr_stream6<double>();
     const bool act = sl[s].phase == PH_REFINE;
     double acc[1] = {0.0};
     if (act)
-        ROWS_UNR(op.D) {
-            ROWS_OF_TRIP(rr)
-            double bv[UNR], ax[UNR];
+        ROWS_UNR_N(op.D, UN) {
+            ROWS_OF_TRIP_N(rr, UN)
+            double bv[UN], ax[UN];
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) bv[u] = rr[u] < op.D ? b[rr[u] * K + s] : 0.0;
-            l_rows<double, K, UNR>(op, rr, s, m, n, x64, te, true, ax);
+            for (int u = 0; u < UN; ++u) bv[u] = rr[u] < op.D ? b[rr[u] * K + s] : 0.0;
+            l_rows<double, K, UN>(op, rr, s, m, n, x64, te, true, ax);
 #pragma unroll
-            for (int u = 0; u < UNR; ++u)
+            for (int u = 0; u < UN; ++u)
                 if (rr[u] < op.D) {
                     const double ri = bv[u] - ax[u];
                     r64[rr[u] * K + s] = ri;
@@ -1535,17 +1545,17 @@ __global__ void __launch_bounds__(BS, 4) k_mixed_start(int64_t D, Slot *sl, Solv
     }
 }
 
-// D^-1 denominators m + n L_rr (src/GeneralizedBiCGStabSystem.h:281-340); identity rows 1
+// D^-1 of D = m + n L_rr (src/GeneralizedBiCGStabSystem.h:281-340); identity rows 1
 template <class T>
-__global__ void k_pden(OpView<T> op, double m, double n, T *__restrict__ pden) {
+__global__ void k_pinv(OpView<T> op, double m, double n, T *__restrict__ pinv) {
     int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (r >= op.D) return;
     if (op.flags[r] & F_IDENT) {
-        pden[r] = (T)1;
+        pinv[r] = (T)1;
         return;
     }
     double ld = (r < op.N) ? (double)op.Ldiag : (double)op.ldiag[r - op.N];
-    pden[r] = (T)(m + ld * n);
+    pinv[r] = (T)(1.0 / (m + ld * n));
 }
 
 // one slot column of a [D][K] array from / to a contiguous vector
@@ -1591,10 +1601,10 @@ struct cpm_solver_s {
     DBuf<double> partial;
     DBuf<unsigned int> counter;
     // FP64 Krylov vectors (plain path) and FP64 refinement state (mixed path)
-    DBuf<double> b64, x64, r64, te64, pden64;
+    DBuf<double> b64, x64, r64, te64, pinv64;
     DBuf<double> dr, dr0, dp, dv, ds, dt, dy, dz;
     // FP32 Krylov vectors of the mixed path
-    DBuf<float> fx, fr, fr0, fp, fv, fs, ft, fy, fz, fte, pden32;
+    DBuf<float> fx, fr, fr0, fp, fv, fs, ft, fy, fz, fte, pinv32;
     bool have64 = false, have32 = false;
     // captured iteration graphs (kernel arguments are fixed pointers; per-solve
     // parameters live in device memory, so a graph is reused while they match)
@@ -1645,7 +1655,7 @@ static void jacobi_rest(cpm_solver_s *s, const SolveParams &P, const double *c, 
     cudaStream_t st = stream();
     for (int j = 1; j < P.sweeps; ++j) {
         launch_epass<double, K>(op, s->slots.p, PH_ITER, y, s->te64.p, st);
-        k_jacobi_sweep<double, K><<<s->G, BS, 0, st>>>(op, s->slots.p, s->m, s->n, c, s->te64.p, s->pden64.p, JACOBI_OMEGA, y);
+        k_jacobi_sweep<double, K><<<s->G, BS, 0, st>>>(op, s->slots.p, s->m, s->n, c, s->te64.p, s->pinv64.p, JACOBI_OMEGA, y);
     }
 }
 
@@ -1655,14 +1665,14 @@ static void plain_iteration(cpm_solver_s *s, const SolveParams &P) {
     const int64_t D = s->D;
     cudaStream_t st = stream();
     Slot *sl = s->slots.p;
-    const double *pden = P.precond == 0 ? nullptr : s->pden64.p;
+    const double *pinv = P.precond == 0 ? nullptr : s->pinv64.p;
     const double ys = P.precond == 2 ? JACOBI_OMEGA : 1.0;
-    k_update_p<double, K><<<s->G, BS, 0, st>>>(D, sl, pden, ys, s->dr.p, s->dv.p, s->dp.p, s->dy.p, s->dr0.p);
+    k_update_p<double, K><<<s->G, BS, 0, st>>>(D, sl, pinv, ys, s->dr.p, s->dv.p, s->dp.p, s->dy.p, s->dr0.p);
     if (P.precond == 2) jacobi_rest<K>(s, P, s->dp.p, s->dy.p);
     launch_epass<double, K>(op, sl, PH_ITER, s->dy.p, s->te64.p, st);
     k_apply_alpha<double, K><<<s->G, BS, 0, st>>>(op, sl, s->m, s->n, s->dy.p, s->te64.p, s->dr0.p, s->dv.p, s->partial.p,
                                                   s->counter.p);
-    k_update_s<double, K><<<s->G, BS, 0, st>>>(D, sl, pden, ys, s->dr.p, s->dv.p, s->ds.p, s->dz.p);
+    k_update_s<double, K><<<s->G, BS, 0, st>>>(D, sl, pinv, ys, s->dr.p, s->dv.p, s->ds.p, s->dz.p);
     if (P.precond == 2) jacobi_rest<K>(s, P, s->ds.p, s->dz.p);
     launch_epass<double, K>(op, sl, PH_ITER, s->dz.p, s->te64.p, st);
     k_apply_omega<double, K><<<s->G, BS, 0, st>>>(op, sl, s->m, s->n, s->dz.p, s->te64.p, s->ds.p, s->dt.p, s->partial.p,
@@ -1687,10 +1697,10 @@ static void mixed_iteration(cpm_solver_s *s, const SolveParams &P) {
     cudaStream_t st = stream();
     Slot *sl = s->slots.p;
     const float m = (float)s->m, n = (float)s->n;
-    const float *pden = P.precond == 0 ? nullptr : s->pden32.p;
+    const float *pinv = P.precond == 0 ? nullptr : s->pinv32.p;
     // four slots per thread: 32 slots, and row offsets D * 32 within 32 bits
     const bool v4 = (K == 32) && D * 32 <= (int64_t)UINT32_MAX;
-    k_update_p<float, K><<<s->G, BS, 0, st>>>(D, sl, pden, 1.0f, s->fr.p, s->fv.p, s->fp.p, s->fy.p, s->fr0.p);
+    k_update_p<float, K><<<s->G, BS, 0, st>>>(D, sl, pinv, 1.0f, s->fr.p, s->fv.p, s->fp.p, s->fy.p, s->fr0.p);
     launch_epass<float, K>(op, sl, PH_ITER, s->fy.p, s->fte.p, st);
     if (v4)
         if (op.ov_ptr)
@@ -1700,7 +1710,7 @@ static void mixed_iteration(cpm_solver_s *s, const SolveParams &P) {
     else
         k_apply_alpha<float, K><<<s->G, BS, 0, st>>>(op, sl, m, n, s->fy.p, s->fte.p, s->fr0.p, s->fv.p, s->partial.p,
                                                      s->counter.p);
-    k_update_s<float, K><<<s->G, BS, 0, st>>>(D, sl, pden, 1.0f, s->fr.p, s->fv.p, s->fs.p, s->fz.p);
+    k_update_s<float, K><<<s->G, BS, 0, st>>>(D, sl, pinv, 1.0f, s->fr.p, s->fv.p, s->fs.p, s->fz.p);
     launch_epass<float, K>(op, sl, PH_ITER, s->fz.p, s->fte.p, st);
     if (v4) {
         if (op.ov_ptr)
@@ -1740,8 +1750,8 @@ static int alloc_vectors(cpm_solver_s *s, bool want64, bool want32) {
     }
     if (want32 && !s->have32) {
         for (auto *b : {&s->fx, &s->fr, &s->fr0, &s->fp, &s->fv, &s->fs, &s->ft, &s->fy, &s->fz, &s->fte}) CPM_TRY(b->alloc(n));
-        CPM_TRY(s->pden32.alloc(s->D));
-        k_pden<float><<<nblk(s->D), BS, 0, stream()>>>(s->op->view<float>(), s->m, s->n, s->pden32.p);
+        CPM_TRY(s->pinv32.alloc(s->D));
+        k_pinv<float><<<nblk(s->D), BS, 0, stream()>>>(s->op->view<float>(), s->m, s->n, s->pinv32.p);
         CPM_CUDA_TRY(cudaGetLastError());
         s->have32 = true;
     }
@@ -2005,10 +2015,10 @@ extern "C" int cpm_solver_create(cpm_opset_t op, double m, double n, int32_t ksl
     if ((rc = s->h_slots.alloc(s->K)) || (rc = s->slots.alloc(s->K)) || (rc = s->partial.alloc((size_t)(s->G + reduce_groups(s->G)) * s->K * 2)) ||
         (rc = s->counter.alloc((size_t)(1 + reduce_groups(s->G)))) ||
         (rc = s->counter.zero()) || (rc = s->b64.alloc((size_t)s->D * s->K)) || (rc = s->x64.alloc((size_t)s->D * s->K)) ||
-        (rc = s->r64.alloc((size_t)s->D * s->K)) || (rc = s->te64.alloc((size_t)s->D * s->K)) || (rc = s->pden64.alloc(s->D)))
+        (rc = s->r64.alloc((size_t)s->D * s->K)) || (rc = s->te64.alloc((size_t)s->D * s->K)) || (rc = s->pinv64.alloc(s->D)))
         return bail(rc);
-    k_pden<double><<<nblk(s->D), BS, 0, stream()>>>(op->view<double>(), m, n, s->pden64.p);
-    if (cudaGetLastError() != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "pden kernel"));
+    k_pinv<double><<<nblk(s->D), BS, 0, stream()>>>(op->view<double>(), m, n, s->pinv64.p);
+    if (cudaGetLastError() != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "pinv kernel"));
     cudaEventCreate(&s->e0);
     cudaEventCreate(&s->e1);
     if (cudaStreamSynchronize(s->own) != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "solver_create"));

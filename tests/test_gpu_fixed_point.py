@@ -43,8 +43,8 @@ def _inputs(kind, n, k, rng):
     return x
 
 
-def _e(op, x):
-    """E~x of [D][k] through the device apply"""
+def _e(op, x, m=0.0, n=-1.0, whole=False):
+    """E~x of [D][k] (whole: and A x) through the device apply"""
     import torch
 
     import cpm_gb300 as cg
@@ -52,10 +52,10 @@ def _e(op, x):
     d = torch.from_numpy(np.ascontiguousarray(x)).cuda()
     t, y = torch.zeros_like(d), torch.zeros_like(d)
     torch.cuda.synchronize()
-    op.apply_device(0.0, -1.0, x.shape[1], False, d.data_ptr(), t.data_ptr(), y.data_ptr())
+    op.apply_device(m, n, x.shape[1], False, d.data_ptr(), t.data_ptr(), y.data_ptr())
     torch.cuda.synchronize()
     cg.sync()
-    return t.cpu().numpy()
+    return (t.cpu().numpy(), y.cpu().numpy()) if whole else t.cpu().numpy()
 
 
 def _reference(rows, x):
@@ -111,3 +111,45 @@ def test_non_finite_values_stay_in_their_rows(op, bad, k):
     assert k == 32 or np.all(fine[~hit])
     assert np.allclose(t[fine, 0], tc[fine, 0], rtol=0, atol=64 * 2.0 ** -52 * 5)
     assert np.array_equal(t[:, 1:], tc[:, 1:])
+
+
+@pytest.mark.parametrize("kind", ["smooth", "rough", "spread", "sparse", "large", "tiny", "low"])
+@pytest.mark.parametrize("k", [1, 32])
+@pytest.mark.parametrize("m,n", [(0.0, -1.0), (1.0, -0.37), (0.5, 0.0), (0.0, 2.0 ** -80)])
+def test_l_rows(op, kind, k, m, n):
+    """A x from the device's own E~x.  The two coefficients, the product with x, the sum's
+    conversion and the result are rounded once each, the FP64 sum of six at most five times:
+    4 units of 2^-52 of |c0 x| + |c1| sum |t|."""
+    op, _ = op
+    rng = np.random.default_rng(5)
+    x = _inputs(kind if kind not in ("large", "low") else "rough", op.D, k, rng)
+    if kind == "large":
+        x *= 2.0 ** 960
+    if kind == "low":  # around the smallest exponent that the row's sum is aligned to
+        x *= np.exp2(rng.integers(-835, -810, x.shape).astype(float))
+    t, y = _e(op, x, m, n, whole=True)
+    ptr, idx, val = op.csr(0)
+    row = np.repeat(np.arange(op.D), np.diff(ptr))
+    ident = op.rows()["identity"]
+    for s in ([0] if k == 1 else [0, 17]):
+        xs, ts = x[:, s].astype(np.longdouble), t[:, s].astype(np.longdouble)
+        diag = idx == row
+        term = np.where(diag, (m + n * val) * xs[idx], n * val * ts[idx])  # m on the diagonal
+        ref = np.where(ident, xs, np.add.reduceat(term, ptr[:-1]))
+        big = np.add.reduceat(np.abs(term), ptr[:-1]).astype(float)
+        err = np.abs((y[:, s] - ref).astype(float))
+        assert np.all(err <= 4 * 2.0 ** -52 * big + 2.0 ** -1070), np.max(err / np.maximum(big, 5e-324)) * 2.0 ** 52
+
+
+@pytest.mark.parametrize("k", [1, 32])
+def test_l_rows_pass_on_non_finite_values(op, k):
+    op, _ = op
+    x = np.random.default_rng(9).standard_normal((op.D, k))
+    x[op.D // 3, 0] = np.inf
+    t, y = _e(op, x, whole=True)
+    ptr, idx, val = op.csr(0)
+    row = np.repeat(np.arange(op.D), np.diff(ptr))
+    ident = op.rows()["identity"]
+    reads = np.where(idx == row, x[idx, 0], t[idx, 0])
+    bad = (np.add.reduceat((~np.isfinite(reads)).astype(int), ptr[:-1]) > 0) & ~ident
+    assert np.array_equal(~np.isfinite(y[:, 0]), bad | (ident & ~np.isfinite(x[:, 0])))
