@@ -131,19 +131,83 @@ struct Dot<float, N> {
     }
 };
 
-// ---- fixed-order grid reduction of NDOT FP64 sums per slot.  Blocks reduce
-// their rows with a tree, groups of RGROUP blocks are summed in block order by
-// the group's last block, and the groups in group order by the last group: the
-// result depends only on the grid size, never on timing or on other slots.
-// partial holds (G + groups) * K * NDOT doubles, counter 1 + groups zeros.
-// SUMMED: the block's per-slot sums are already in v of threads tid < K (the
-// other threads' v are not read), and the block tree is skipped.
+// ---- fixed-order grid reductions of NDOT FP64 sums per slot: the result depends
+// only on the grid size, never on timing or on other slots.  A block's arrival is
+// one thread's fence and counter, ordered after the writes of its own warp.
+__device__ __forceinline__ bool arrive_last(unsigned int *counter, unsigned n) {
+    __threadfence();
+    const bool last = atomicAdd(counter, 1u) == n - 1;
+    __threadfence();
+    return last;
+}
+
+// sums of a block's BS values by a tree, in thread 0.  The FP64 units take 19
+// clocks a warp, so the tree halves the warps that add (12 warp additions) rather
+// than shuffling in all eight (40).
+template <int NDOT>
+__device__ __forceinline__ void block_tree(double (&v)[NDOT], double (&sh)[NDOT][BS]) {
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int d = 0; d < NDOT; ++d) sh[d][tid] = v[d];
+#pragma unroll
+    for (int h = BS / 2; h >= 32; h >>= 1) {
+        __syncthreads();
+        if (tid < h)
+#pragma unroll
+            for (int d = 0; d < NDOT; ++d) {
+                v[d] += sh[d][tid + h];
+                if (h > 32) sh[d][tid] = v[d];
+            }
+    }
+    if (tid < 32)
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1)
+#pragma unroll
+            for (int d = 0; d < NDOT; ++d) v[d] += __shfl_down_sync(FULL, v[d], h);
+}
+
+// one slot: at most four blocks an SM leave a sum each, the last block adds them
+// (thread i those of blocks i, i + BS, ..., then the tree).  With two levels of
+// counters and eight-barrier trees the reduction was 8 of the 12 us of a dot
+// product's kernel on 22 thousand rows.  partial holds G * NDOT doubles.
+template <int NDOT>
+__device__ __forceinline__ bool grid_reduce1(double (&v)[NDOT], double *partial, unsigned int *counter, double (&out)[NDOT]) {
+    __shared__ double sh[NDOT][BS];
+    __shared__ bool last;
+    const int tid = threadIdx.x;
+    const unsigned G = gridDim.x;
+    block_tree<NDOT>(v, sh);
+    if (tid == 0) {
+#pragma unroll
+        for (int d = 0; d < NDOT; ++d) partial[(size_t)blockIdx.x * NDOT + d] = v[d];
+        last = arrive_last(counter, G);
+    }
+    __syncthreads();
+    if (!last) return false;
+#pragma unroll
+    for (int d = 0; d < NDOT; ++d) out[d] = 0.0;
+    for (unsigned b = tid; b < G; b += BS)
+#pragma unroll
+        for (int d = 0; d < NDOT; ++d) out[d] += __ldcg(partial + (size_t)b * NDOT + d);
+    block_tree<NDOT>(out, sh);
+    if (tid == 0) *counter = 0u;
+    return tid == 0;
+}
+
+// K slots: blocks reduce their rows with a tree, groups of RGROUP blocks are
+// summed in block order by the group's last block, and the groups in group order
+// by the last group (all blocks' sums of 32 slots in one block would take its FP64
+// units 12 us).  partial holds (G + groups) * K * NDOT doubles, counter 1 + groups
+// zeros.  SUMMED: the block's per-slot sums are already in v of threads tid < K
+// (the other threads' v are not read), and the block tree is skipped.
 template <int K, int NDOT, bool SUMMED = false>
 __device__ __forceinline__ bool grid_reduce(double (&v)[NDOT], double *partial, unsigned int *counter, double (&out)[NDOT]) {
+    if constexpr (K == 1 && !SUMMED) return grid_reduce1<NDOT>(v, partial, counter, out);
     __shared__ double sh[NDOT][BS];
     __shared__ bool last;
     const int tid = threadIdx.x;
     constexpr int RPB = BS / K;
+    static_assert(K == 1 || K == 32, "the slots' threads are one warp");
     const int slot = tid % K, chunk = tid / K;
     auto tree = [&]() {
         __syncthreads();
@@ -158,7 +222,6 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NDOT], double *partial, 
         if (tid < K)
 #pragma unroll
             for (int d = 0; d < NDOT; ++d) sh[d][tid] = v[d];
-        __syncthreads();
     } else {
 #pragma unroll
         for (int d = 0; d < NDOT; ++d) sh[d][tid] = v[d];
@@ -166,16 +229,15 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NDOT], double *partial, 
     }
     const unsigned G = gridDim.x, grp = blockIdx.x / RGROUP, ngrp = (G + RGROUP - 1) / RGROUP;
     double *gpart = partial + (size_t)G * K * NDOT;
-    if (tid < K)
+    const unsigned b0 = grp * RGROUP, b1 = min(b0 + RGROUP, G);
+    if (tid < K) {
 #pragma unroll
         for (int d = 0; d < NDOT; ++d) partial[((size_t)blockIdx.x * K + tid) * NDOT + d] = sh[d][tid];
-    __threadfence();
-    __syncthreads();
-    const unsigned b0 = grp * RGROUP, b1 = min(b0 + RGROUP, G);
-    if (tid == 0) last = (atomicAdd(counter + 1 + grp, 1u) == b1 - b0 - 1);
+        __syncwarp();
+        if (tid == 0) last = arrive_last(counter + 1 + grp, b1 - b0);
+    }
     __syncthreads();
     if (!last) return false;
-    __threadfence();
     double acc[NDOT];
 #pragma unroll
     for (int d = 0; d < NDOT; ++d) acc[d] = 0.0;
@@ -189,16 +251,17 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NDOT], double *partial, 
 #pragma unroll
     for (int d = 0; d < NDOT; ++d) sh[d][tid] = acc[d];
     tree();
-    if (tid < K)
+    if (tid < K) {
 #pragma unroll
         for (int d = 0; d < NDOT; ++d) gpart[((size_t)grp * K + tid) * NDOT + d] = sh[d][tid];
-    if (tid == 0) counter[1 + grp] = 0u;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) last = (atomicAdd(counter, 1u) == ngrp - 1);
+        __syncwarp();
+        if (tid == 0) {
+            counter[1 + grp] = 0u;
+            last = arrive_last(counter, ngrp);
+        }
+    }
     __syncthreads();
     if (!last) return false;
-    __threadfence();
 #pragma unroll
     for (int d = 0; d < NDOT; ++d) acc[d] = 0.0;
     for (unsigned g = chunk; g < ngrp; g += RPB)
