@@ -88,6 +88,32 @@ static inline int row_grid(int64_t D, int K) {
 }
 static inline int64_t reduce_groups(int G) { return (G + RGROUP - 1) / RGROUP; }
 
+// ---- dependent launches.  The kernels of the iterations and applies are launched
+// so that a kernel's blocks are placed, and its operator tables read, while the
+// previous one drains: a launch otherwise costs 1 to 2 us between kernels that
+// take 3 to 20 us.  Each begins with pdl_wait(), before it reads or writes
+// anything another kernel writes, in every block: it returns once the previous
+// kernel is complete and its writes are visible, so completion is transitive.
+// Vectors that a previous kernel writes are not __restrict__ there: a read-only
+// load may not be issued before the wait.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+static void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // ---- per-thread dot products.  FP64 vectors accumulate in FP64.  FP32 vectors
 // accumulate in a double-float pair on the FP32 pipes (FP64 units are scarce on
 // this GPU): each product a*b is split exactly into p + e by an FMA, p is added
@@ -400,8 +426,9 @@ __device__ __forceinline__ void e_ident32(const OpView<T> &op, int warp, int lan
 // time; weights staged pair-interleaved in the warp's shared memory.  Identity
 // rows copied warp per row.  ph < 0: every slot.
 constexpr int EW_ROWS = 8;
-__global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *__restrict__ sl, int ph, int nb_plain,
-                                                  const float *__restrict__ x, float *__restrict__ t) {
+__global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *sl, int ph, int nb_plain,
+                                                  const float *x, float *t) {
+    pdl_wait();
     __shared__ __align__(16) float sw[4][EW_ROWS * 12];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool act = (ph < 0) || sl[lane].phase == ph;
@@ -510,8 +537,9 @@ __device__ __forceinline__ bool fx_out(uint32_t e20) { return e20 - FX_EMIN >= F
 // and the pass took 435 us on the two-circle sphere at dx 0.025.)  The rows'
 // weights are broadcast from shared memory.
 constexpr int EX_ROWS = 8;
-__global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Slot *__restrict__ sl, int ph, int nb_plain,
-                                                     const double *__restrict__ x, double *__restrict__ t) {
+__global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Slot *sl, int ph, int nb_plain,
+                                                     const double *x, double *t) {
+    pdl_wait();
     __shared__ __align__(16) int2 sw[4][EX_ROWS * 12];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane >> 4, s = (lane & 15) + 16 * (warp & 1);
     const bool act32 = (ph < 0) || sl[lane].phase == ph;
@@ -656,44 +684,50 @@ __device__ __forceinline__ double e1_row(const OpView<double> &op, int64_t p, ui
 }
 
 template <class T>
-__global__ void __launch_bounds__(E1_T) k_epass1(OpView<T> op, const Slot *__restrict__ sl, int ph, unsigned row_blocks,
-                                                 const T *__restrict__ x, T *__restrict__ t) {
+__global__ void __launch_bounds__(E1_T, 7) k_epass1(OpView<T> op, const Slot *sl, int ph, unsigned row_blocks,
+                                                 const T *x, T *t) {
     __shared__ E1Group<T> sh[E1_T / 32][E1_GROUPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * (E1_T / 32) + warp;
+    const bool rows = blockIdx.x < row_blocks && c < op.n_chunk;
+    // the operator's own tables while the previous kernel ends
+    int4 ch = make_int4(0, 0, 0, 0);
+    int ca[E1_GROUPS], cb[E1_GROUPS], r = 0;
+    uint8_t fl = 0;
+    int64_t p = 0;
+    if (rows) {
+        ch = __ldg(op.chunk + c);
+        const int32_t *gc = op.gcols + 64 * (int64_t)ch.x + lane;
+#pragma unroll
+        for (int g = 0; g < E1_GROUPS; ++g)
+            if (g < ch.w >> 8) {
+                ca[g] = __ldg(gc + 64 * g);
+                cb[g] = __ldg(gc + 64 * g + 32);
+            }
+        p = ch.y + min(lane, (ch.w & 255) - 1);
+        r = __ldg(op.ord + p);
+        fl = __ldg(op.fl_ord + p) & F_TERMS;
+    }
+    pdl_wait();
     if (ph >= 0 && sl[0].phase != ph) return;
     if (blockIdx.x >= row_blocks) {  // identity rows
         const int64_t q = (int64_t)(blockIdx.x - row_blocks) * E1_T + threadIdx.x;
         if (q < op.n_ident) {
-            const int r = op.ident[q];
-            t[r] = x[r];
+            const int ri = op.ident[q];
+            t[ri] = x[ri];
         }
         return;
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t c = (int64_t)blockIdx.x * (E1_T / 32) + warp;
-    if (c >= op.n_chunk) return;
-    const int4 ch = __ldg(op.chunk + c);
+    if (!rows) return;
     const int ng = ch.w >> 8, nr = ch.w & 255;
-    const int32_t *gc = op.gcols + 64 * (int64_t)ch.x + lane;
     T xa[E1_GROUPS], xb[E1_GROUPS];
-    {
-        int ca[E1_GROUPS], cb[E1_GROUPS];
 #pragma unroll
-        for (int g = 0; g < E1_GROUPS; ++g)
-            if (g < ng) {
-                ca[g] = __ldg(gc + 64 * g);
-                cb[g] = __ldg(gc + 64 * g + 32);
-            }
-#pragma unroll
-        for (int g = 0; g < E1_GROUPS; ++g)
-            if (g < ng) {
-                xa[g] = x[ca[g]];
-                xb[g] = x[cb[g]];
-            }
-    }
-    const int64_t p = ch.y + min(lane, nr - 1);
+    for (int g = 0; g < E1_GROUPS; ++g)
+        if (g < ng) {
+            xa[g] = x[ca[g]];
+            xb[g] = x[cb[g]];
+        }
     const int mine = __popc((uint32_t)ch.z & (0xffffffffu >> (31 - lane))) - 1;  // the row's group
-    const int r = __ldg(op.ord + p);
-    const uint8_t fl = __ldg(op.fl_ord + p) & F_TERMS;
     uint32_t e20 = FX_EMIN;  // exponent field of the row's group
     bool zero = false;       // the warp's groups of smallest exponent hold zeros only
     if constexpr (sizeof(T) == 8) {
@@ -735,8 +769,9 @@ __global__ void __launch_bounds__(E1_T) k_epass1(OpView<T> op, const Slot *__res
 // after the bulk E pass: warp per row with records, lane = slot,
 // t += sum over the slot's E entries of w (x[DOF column] - x[replaced column])
 template <class T>
-__global__ void __launch_bounds__(128) k_slot_epatch32(OpView<T> op, const Slot *__restrict__ sl, int ph, const T *__restrict__ x,
-                                                       T *__restrict__ t) {
+__global__ void __launch_bounds__(128) k_slot_epatch32(OpView<T> op, const Slot *sl, int ph, const T *x,
+                                                       T *t) {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const bool act = (ph < 0) || sl[lane].phase == ph;
     if (!__any_sync(FULL, act)) return;
@@ -759,7 +794,7 @@ __global__ void __launch_bounds__(128) k_slot_epatch32(OpView<T> op, const Slot 
 template <class T>
 static void slot_epatch(const OpView<T> &op, const Slot *sl, int ph, const T *x, T *t, cudaStream_t st) {
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((op.n_sp_rows + 3) / 4, 16LL * sm_count()));
-    k_slot_epatch32<T><<<(unsigned)blocks, 128, 0, st>>>(op, sl, ph, x, t);
+    launch_after(k_slot_epatch32<T>, (unsigned)blocks, 128, st, op, sl, ph, x, t);
 }
 
 // default launch shapes of the 32-slot E passes (blocks per SM caps of the
@@ -788,12 +823,12 @@ static void launch_epass(const OpView<T> &op, const Slot *sl, int ph, const T *x
         const int crossing = group_blocks<T>(op.n_grp - op.n_grp_plain, op.patch_bps > 0 ? op.patch_bps : PATCH_BPS);
         const unsigned blocks = (unsigned)std::max(1, plain + crossing);
         if constexpr (sizeof(T) == 4)
-            k_epass32w<<<blocks, 128, 0, st>>>(op, sl, ph, plain, x, t);
+            launch_after(k_epass32w, blocks, 128, st, op, sl, ph, plain, x, t);
         else
-            k_epass32x<<<blocks, 128, 0, st>>>(op, sl, ph, plain, x, t);
+            launch_after(k_epass32x, blocks, 128, st, op, sl, ph, plain, x, t);
     } else {
         const unsigned rows = (unsigned)((op.n_chunk + E1_T / 32 - 1) / (E1_T / 32)), id = (unsigned)((op.n_ident + E1_T - 1) / E1_T);
-        k_epass1<T><<<std::max(1u, rows + id), E1_T, 0, st>>>(op, sl, ph, rows, x, t);
+        launch_after(k_epass1<T>, std::max(1u, rows + id), E1_T, st, op, sl, ph, rows, x, t);
     }
     if (K == 32 && op.n_sp_rows > 0) slot_epatch(op, sl, ph, x, t, st);
 }
@@ -829,8 +864,9 @@ constexpr int unr_stream6() { return sizeof(T) == 8 ? 2 : UNR; }
 
 // y = m x + n (Ldiag x + Loff E~-gathered neighbours): the L pass of one apply
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_lpass(OpView<T> op, T m, T n, const T *__restrict__ x, const T *__restrict__ t,
-                                              T *__restrict__ y) {
+__global__ void __launch_bounds__(BS, 4) k_lpass(OpView<T> op, T m, T n, const T *x, const T *t,
+                                              T *y) {
+    pdl_wait();
     GRID_LOOP
     constexpr int UN = unr_stream6<T>();
     ROWS_UNR_N(op.D, UN) {
@@ -925,9 +961,10 @@ __global__ void __launch_bounds__(BS, 4) k_init(OpView<T> op, Slot *sl, SolvePar
 // rounding of M^-1 does not enter x, which is updated by the y that A was applied to.
 // (src/GeneralizedBiCGStabSystem.h:358-377 with result = 0 and A 0 = 0)
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_update_p(int64_t D, const Slot *__restrict__ sl, const T *__restrict__ pinv, T ys,
-                                                 const T *__restrict__ r, const T *__restrict__ v, T *__restrict__ p,
-                                                 T *__restrict__ y, T *__restrict__ r0) {
+__global__ void __launch_bounds__(BS, 4) k_update_p(int64_t D, const Slot *sl, const T *pinv, T ys,
+                                                 const T *r, const T *v, T *p,
+                                                 T *y, T *r0) {
+    pdl_wait();
     GRID_LOOP
     constexpr int UN = unr_stream6<T>();
     if (sl[s].phase != PH_ITER) return;
@@ -964,9 +1001,10 @@ __global__ void __launch_bounds__(BS, 4) k_update_p(int64_t D, const Slot *__res
 
 // v = A y with r0 . v  ->  alpha = rho / (r0 . v)   (src/BiCGStab.h:79-80)
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_apply_alpha(OpView<T> op, Slot *sl, T m, T n, const T *__restrict__ y,
-                                                    const T *__restrict__ te, const T *__restrict__ r0, T *__restrict__ v,
+__global__ void __launch_bounds__(BS, 4) k_apply_alpha(OpView<T> op, Slot *sl, T m, T n, const T *y,
+                                                    const T *te, const T *r0, T *v,
                                                     double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP
     constexpr int UN = unr_stream6<T>();
     const bool act = sl[s].phase == PH_ITER;
@@ -992,9 +1030,10 @@ __global__ void __launch_bounds__(BS, 4) k_apply_alpha(OpView<T> op, Slot *sl, T
 
 // s = r - alpha v ; z = M^-1 s   (src/BiCGStab.h:82-84), M^-1 as in k_update_p
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_update_s(int64_t D, const Slot *__restrict__ sl, const T *__restrict__ pinv, T ys,
-                                                 const T *__restrict__ r, const T *__restrict__ v, T *__restrict__ sv,
-                                                 T *__restrict__ z) {
+__global__ void __launch_bounds__(BS, 4) k_update_s(int64_t D, const Slot *sl, const T *pinv, T ys,
+                                                 const T *r, const T *v, T *sv,
+                                                 T *z) {
+    pdl_wait();
     GRID_LOOP
     if (sl[s].phase != PH_ITER) return;
     const T a = (T)sl[s].alpha;
@@ -1024,9 +1063,10 @@ __global__ void __launch_bounds__(BS, 4) k_update_s(int64_t D, const Slot *__res
 // y += omega ((c - A y) pinv)   (src/GeneralizedBiCGStabSystem.h:366-376).
 // Row r of A y reads y only at row r, so the update is in place.
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_jacobi_sweep(OpView<T> op, const Slot *__restrict__ sl, T m, T n,
-                                                     const T *__restrict__ c, const T *__restrict__ te,
-                                                     const T *__restrict__ pinv, T omega, T *y) {
+__global__ void __launch_bounds__(BS, 4) k_jacobi_sweep(OpView<T> op, const Slot *sl, T m, T n,
+                                                     const T *c, const T *te,
+                                                     const T *pinv, T omega, T *y) {
+    pdl_wait();
     GRID_LOOP
     constexpr int UN = unr_stream6<T>();
     if (sl[s].phase != PH_ITER) return;
@@ -1051,9 +1091,10 @@ __global__ void __launch_bounds__(BS, 4) k_jacobi_sweep(OpView<T> op, const Slot
 
 // t = A z with t.t and t.s  ->  omega   (src/BiCGStab.h:85-95)
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_apply_omega(OpView<T> op, Slot *sl, T m, T n, const T *__restrict__ z,
-                                                    const T *__restrict__ te, const T *__restrict__ sv, T *__restrict__ tv,
+__global__ void __launch_bounds__(BS, 4) k_apply_omega(OpView<T> op, Slot *sl, T m, T n, const T *z,
+                                                    const T *te, const T *sv, T *tv,
                                                     double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP
     constexpr int UN = unr_stream6<T>();
     const bool act = sl[s].phase == PH_ITER;
@@ -1081,10 +1122,11 @@ __global__ void __launch_bounds__(BS, 4) k_apply_omega(OpView<T> op, Slot *sl, T
 // x += alpha y + w z ; r = s - w t ; r.r and r0.r -> convergence test, rho, beta
 // (src/BiCGStab.h:97-103 and the loop head :59-73)
 template <class T, int K>
-__global__ void __launch_bounds__(BS, 4) k_update_xr(int64_t D, Slot *sl, SolveParams P, const T *__restrict__ y,
-                                                  const T *__restrict__ z, const T *__restrict__ sv,
-                                                  const T *__restrict__ tv, const T *__restrict__ r0, T *__restrict__ x,
-                                                  T *__restrict__ r, double *partial, unsigned int *counter) {
+__global__ void __launch_bounds__(BS, 4) k_update_xr(int64_t D, Slot *sl, SolveParams P, const T *y,
+                                                  const T *z, const T *sv,
+                                                  const T *tv, const T *r0, T *x,
+                                                  T *r, double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP
     const bool act = sl[s].phase == PH_ITER;
     Dot<T, 2> acc;
@@ -1258,8 +1300,9 @@ __device__ __forceinline__ bool grid_reduce4(const Dot4<N> &acc, double *partial
 
 // k_lpass for 32 FP32 slots (every slot); OVL as in l_rows4
 template <bool OVL>
-__global__ void __launch_bounds__(BS, 4) k_lpass4(OpView<float> op, float m, float n, const float *__restrict__ x,
-                                               const float *__restrict__ t, float *__restrict__ y) {
+__global__ void __launch_bounds__(BS, 4) k_lpass4(OpView<float> op, float m, float n, const float *x,
+                                               const float *t, float *y) {
+    pdl_wait();
     GRID_LOOP4
     ROWS4(op.D, V4_UN) {
         ROWS4_OF_TRIP(rr, V4_UN)
@@ -1279,9 +1322,10 @@ static inline bool lpass4_ok(int64_t D, const void *a, const void *b, const void
 
 // k_apply_alpha for 32 FP32 slots
 template <bool OVL>
-__global__ void __launch_bounds__(BS, 4) k_apply_alpha4(OpView<float> op, Slot *sl, float m, float n, const float *__restrict__ y,
-                                                     const float *__restrict__ te, const float *__restrict__ r0,
-                                                     float *__restrict__ v, double *partial, unsigned int *counter) {
+__global__ void __launch_bounds__(BS, 4) k_apply_alpha4(OpView<float> op, Slot *sl, float m, float n, const float *y,
+                                                     const float *te, const float *r0,
+                                                     float *v, double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP4
     const unsigned act = act4(sl, q, PH_ITER);
     uint64_t m0, m1;
@@ -1307,9 +1351,10 @@ __global__ void __launch_bounds__(BS, 4) k_apply_alpha4(OpView<float> op, Slot *
 
 // k_apply_omega for 32 FP32 slots
 template <bool OVL>
-__global__ void __launch_bounds__(BS, 4) k_apply_omega4(OpView<float> op, Slot *sl, float m, float n, const float *__restrict__ z,
-                                                     const float *__restrict__ te, const float *__restrict__ sv,
-                                                     float *__restrict__ tv, double *partial, unsigned int *counter) {
+__global__ void __launch_bounds__(BS, 4) k_apply_omega4(OpView<float> op, Slot *sl, float m, float n, const float *z,
+                                                     const float *te, const float *sv,
+                                                     float *tv, double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP4
     const unsigned act = act4(sl, q, PH_ITER);
     uint64_t m0, m1;
@@ -1335,10 +1380,11 @@ __global__ void __launch_bounds__(BS, 4) k_apply_omega4(OpView<float> op, Slot *
 }
 
 // k_update_xr for 32 FP32 slots
-__global__ void __launch_bounds__(BS, 4) k_update_xr4(int64_t D, Slot *sl, SolveParams P, const float *__restrict__ y,
-                                                   const float *__restrict__ z, const float *__restrict__ sv,
-                                                   const float *__restrict__ tv, const float *__restrict__ r0, float *x,
-                                                   float *__restrict__ r, double *partial, unsigned int *counter) {
+__global__ void __launch_bounds__(BS, 4) k_update_xr4(int64_t D, Slot *sl, SolveParams P, const float *y,
+                                                   const float *z, const float *sv,
+                                                   const float *tv, const float *r0, float *x,
+                                                   float *r, double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP4
     const unsigned act = act4(sl, q, PH_ITER);
     uint64_t m0, m1;
@@ -1427,6 +1473,7 @@ __global__ void __launch_bounds__(BS, 4) k_restart(OpView<T> op, Slot *sl, T m, 
 // otherwise never meet the true residual, nor the stagnation exit)
 template <int K>
 __global__ void k_refine_gate(Slot *sl, SolveParams P) {
+    pdl_wait();
     const int s = threadIdx.x;
     if (s >= K) return;
     Slot &S = sl[s];
@@ -1436,7 +1483,8 @@ __global__ void k_refine_gate(Slot *sl, SolveParams P) {
 
 // reliable update, step 1: x64 += scale * u32, u32 = 0
 template <int K>
-__global__ void k_refine_accumulate(int64_t D, const Slot *__restrict__ sl, float *__restrict__ u, double *__restrict__ x64) {
+__global__ void k_refine_accumulate(int64_t D, const Slot *sl, float *u, double *x64) {
+    pdl_wait();
     int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t row = gid / K;
     int s = (int)(gid % K);
@@ -1448,9 +1496,10 @@ __global__ void k_refine_accumulate(int64_t D, const Slot *__restrict__ sl, floa
 // step 2: r64 = b - A x64 (FP64) and ||r64||: done, or replace the FP32 residual
 template <int K>
 __global__ void __launch_bounds__(BS, 4) k_refine_residual(OpView<double> op, Slot *sl, SolveParams P, double m, double n,
-                                                        const double *__restrict__ b, const double *__restrict__ x64,
-                                                        const double *__restrict__ te, double *__restrict__ r64,
+                                                        const double *b, const double *x64,
+                                                        const double *te, double *r64,
                                                         double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP
     constexpr int UN = unr_stream6<double>();
     const bool act = sl[s].phase == PH_REFINE;
@@ -1500,9 +1549,10 @@ __global__ void __launch_bounds__(BS, 4) k_refine_residual(OpView<double> op, Sl
 // step 3: r32 = r64 / scale; keep p, v, r0 and the scalars, recompute rho = r0 . r
 // (after a rho breakdown the Krylov space restarts from the true residual instead)
 template <int K>
-__global__ void __launch_bounds__(BS, 4) k_reliable(int64_t D, Slot *sl, const double *__restrict__ r64, float *__restrict__ r,
-                                                 float *__restrict__ r0, float *__restrict__ p, float *__restrict__ v,
+__global__ void __launch_bounds__(BS, 4) k_reliable(int64_t D, Slot *sl, const double *r64, float *r,
+                                                 float *r0, float *p, float *v,
                                                  double *partial, unsigned int *counter) {
+    pdl_wait();
     GRID_LOOP
     const bool act = sl[s].phase == PH_RELIABLE;
     const bool fresh = act && sl[s].krylov_restart;
@@ -1718,7 +1768,7 @@ static void jacobi_rest(cpm_solver_s *s, const SolveParams &P, const double *c, 
     cudaStream_t st = stream();
     for (int j = 1; j < P.sweeps; ++j) {
         launch_epass<double, K>(op, s->slots.p, PH_ITER, y, s->te64.p, st);
-        k_jacobi_sweep<double, K><<<s->G, BS, 0, st>>>(op, s->slots.p, s->m, s->n, c, s->te64.p, s->pinv64.p, JACOBI_OMEGA, y);
+        launch_after(k_jacobi_sweep<double, K>, s->G, BS, st, op, s->slots.p, s->m, s->n, c, s->te64.p, s->pinv64.p, JACOBI_OMEGA, y);
     }
 }
 
@@ -1730,17 +1780,17 @@ static void plain_iteration(cpm_solver_s *s, const SolveParams &P) {
     Slot *sl = s->slots.p;
     const double *pinv = P.precond == 0 ? nullptr : s->pinv64.p;
     const double ys = P.precond == 2 ? JACOBI_OMEGA : 1.0;
-    k_update_p<double, K><<<s->G, BS, 0, st>>>(D, sl, pinv, ys, s->dr.p, s->dv.p, s->dp.p, s->dy.p, s->dr0.p);
+    launch_after(k_update_p<double, K>, s->G, BS, st, D, sl, pinv, ys, s->dr.p, s->dv.p, s->dp.p, s->dy.p, s->dr0.p);
     if (P.precond == 2) jacobi_rest<K>(s, P, s->dp.p, s->dy.p);
     launch_epass<double, K>(op, sl, PH_ITER, s->dy.p, s->te64.p, st);
-    k_apply_alpha<double, K><<<s->G, BS, 0, st>>>(op, sl, s->m, s->n, s->dy.p, s->te64.p, s->dr0.p, s->dv.p, s->partial.p,
+    launch_after(k_apply_alpha<double, K>, s->G, BS, st, op, sl, s->m, s->n, s->dy.p, s->te64.p, s->dr0.p, s->dv.p, s->partial.p,
                                                   s->counter.p);
-    k_update_s<double, K><<<s->G, BS, 0, st>>>(D, sl, pinv, ys, s->dr.p, s->dv.p, s->ds.p, s->dz.p);
+    launch_after(k_update_s<double, K>, s->G, BS, st, D, sl, pinv, ys, s->dr.p, s->dv.p, s->ds.p, s->dz.p);
     if (P.precond == 2) jacobi_rest<K>(s, P, s->ds.p, s->dz.p);
     launch_epass<double, K>(op, sl, PH_ITER, s->dz.p, s->te64.p, st);
-    k_apply_omega<double, K><<<s->G, BS, 0, st>>>(op, sl, s->m, s->n, s->dz.p, s->te64.p, s->ds.p, s->dt.p, s->partial.p,
+    launch_after(k_apply_omega<double, K>, s->G, BS, st, op, sl, s->m, s->n, s->dz.p, s->te64.p, s->ds.p, s->dt.p, s->partial.p,
                                                   s->counter.p);
-    k_update_xr<double, K><<<s->G, BS, 0, st>>>(D, sl, P, s->dy.p, s->dz.p, s->ds.p, s->dt.p, s->dr0.p, s->x64.p, s->dr.p,
+    launch_after(k_update_xr<double, K>, s->G, BS, st, D, sl, P, s->dy.p, s->dz.p, s->ds.p, s->dt.p, s->dr0.p, s->x64.p, s->dr.p,
                                                 s->partial.p, s->counter.p);
 }
 
@@ -1763,29 +1813,29 @@ static void mixed_iteration(cpm_solver_s *s, const SolveParams &P) {
     const float *pinv = P.precond == 0 ? nullptr : s->pinv32.p;
     // four slots per thread: 32 slots, and row offsets D * 32 within 32 bits
     const bool v4 = (K == 32) && D * 32 <= (int64_t)UINT32_MAX;
-    k_update_p<float, K><<<s->G, BS, 0, st>>>(D, sl, pinv, 1.0f, s->fr.p, s->fv.p, s->fp.p, s->fy.p, s->fr0.p);
+    launch_after(k_update_p<float, K>, s->G, BS, st, D, sl, pinv, 1.0f, s->fr.p, s->fv.p, s->fp.p, s->fy.p, s->fr0.p);
     launch_epass<float, K>(op, sl, PH_ITER, s->fy.p, s->fte.p, st);
     if (v4)
         if (op.ov_ptr)
-            k_apply_alpha4<true><<<s->G, BS, 0, st>>>(op, sl, m, n, s->fy.p, s->fte.p, s->fr0.p, s->fv.p, s->partial.p, s->counter.p);
+            launch_after(k_apply_alpha4<true>, s->G, BS, st, op, sl, m, n, s->fy.p, s->fte.p, s->fr0.p, s->fv.p, s->partial.p, s->counter.p);
         else
-            k_apply_alpha4<false><<<s->G, BS, 0, st>>>(op, sl, m, n, s->fy.p, s->fte.p, s->fr0.p, s->fv.p, s->partial.p, s->counter.p);
+            launch_after(k_apply_alpha4<false>, s->G, BS, st, op, sl, m, n, s->fy.p, s->fte.p, s->fr0.p, s->fv.p, s->partial.p, s->counter.p);
     else
-        k_apply_alpha<float, K><<<s->G, BS, 0, st>>>(op, sl, m, n, s->fy.p, s->fte.p, s->fr0.p, s->fv.p, s->partial.p,
+        launch_after(k_apply_alpha<float, K>, s->G, BS, st, op, sl, m, n, s->fy.p, s->fte.p, s->fr0.p, s->fv.p, s->partial.p,
                                                      s->counter.p);
-    k_update_s<float, K><<<s->G, BS, 0, st>>>(D, sl, pinv, 1.0f, s->fr.p, s->fv.p, s->fs.p, s->fz.p);
+    launch_after(k_update_s<float, K>, s->G, BS, st, D, sl, pinv, 1.0f, s->fr.p, s->fv.p, s->fs.p, s->fz.p);
     launch_epass<float, K>(op, sl, PH_ITER, s->fz.p, s->fte.p, st);
     if (v4) {
         if (op.ov_ptr)
-            k_apply_omega4<true><<<s->G, BS, 0, st>>>(op, sl, m, n, s->fz.p, s->fte.p, s->fs.p, s->ft.p, s->partial.p, s->counter.p);
+            launch_after(k_apply_omega4<true>, s->G, BS, st, op, sl, m, n, s->fz.p, s->fte.p, s->fs.p, s->ft.p, s->partial.p, s->counter.p);
         else
-            k_apply_omega4<false><<<s->G, BS, 0, st>>>(op, sl, m, n, s->fz.p, s->fte.p, s->fs.p, s->ft.p, s->partial.p, s->counter.p);
-        k_update_xr4<<<s->G, BS, 0, st>>>(D, sl, P, s->fy.p, s->fz.p, s->fs.p, s->ft.p, s->fr0.p, s->fx.p, s->fr.p,
+            launch_after(k_apply_omega4<false>, s->G, BS, st, op, sl, m, n, s->fz.p, s->fte.p, s->fs.p, s->ft.p, s->partial.p, s->counter.p);
+        launch_after(k_update_xr4, s->G, BS, st, D, sl, P, s->fy.p, s->fz.p, s->fs.p, s->ft.p, s->fr0.p, s->fx.p, s->fr.p,
                                           s->partial.p, s->counter.p);
     } else {
-        k_apply_omega<float, K><<<s->G, BS, 0, st>>>(op, sl, m, n, s->fz.p, s->fte.p, s->fs.p, s->ft.p, s->partial.p,
+        launch_after(k_apply_omega<float, K>, s->G, BS, st, op, sl, m, n, s->fz.p, s->fte.p, s->fs.p, s->ft.p, s->partial.p,
                                                      s->counter.p);
-        k_update_xr<float, K><<<s->G, BS, 0, st>>>(D, sl, P, s->fy.p, s->fz.p, s->fs.p, s->ft.p, s->fr0.p, s->fx.p, s->fr.p,
+        launch_after(k_update_xr<float, K>, s->G, BS, st, D, sl, P, s->fy.p, s->fz.p, s->fs.p, s->ft.p, s->fr0.p, s->fx.p, s->fr.p,
                                                    s->partial.p, s->counter.p);
     }
 }
@@ -1797,12 +1847,12 @@ static void mixed_refine(cpm_solver_s *s, const SolveParams &P) {
     const int64_t D = s->D;
     cudaStream_t st = stream();
     Slot *sl = s->slots.p;
-    k_refine_gate<K><<<1, 32, 0, st>>>(sl, P);
-    k_refine_accumulate<K><<<nblk(D * K), BS, 0, st>>>(D, sl, s->fx.p, s->x64.p);
+    launch_after(k_refine_gate<K>, 1, 32, st, sl, P);
+    launch_after(k_refine_accumulate<K>, nblk(D * K), BS, st, D, sl, s->fx.p, s->x64.p);
     launch_epass<double, K>(op64, sl, PH_REFINE, s->x64.p, s->te64.p, st);
-    k_refine_residual<K><<<s->G, BS, 0, st>>>(op64, sl, P, s->m, s->n, s->b64.p, s->x64.p, s->te64.p, s->r64.p, s->partial.p,
+    launch_after(k_refine_residual<K>, s->G, BS, st, op64, sl, P, s->m, s->n, s->b64.p, s->x64.p, s->te64.p, s->r64.p, s->partial.p,
                                               s->counter.p);
-    k_reliable<K><<<s->G, BS, 0, st>>>(D, sl, s->r64.p, s->fr.p, s->fr0.p, s->fp.p, s->fv.p, s->partial.p, s->counter.p);
+    launch_after(k_reliable<K>, s->G, BS, st, D, sl, s->r64.p, s->fr.p, s->fr0.p, s->fp.p, s->fv.p, s->partial.p, s->counter.p);
 }
 
 static int alloc_vectors(cpm_solver_s *s, bool want64, bool want32) {
@@ -2482,7 +2532,7 @@ extern "C" int cpm_apply(cpm_opset_t op, double m, double n, int32_t k, const do
     for (int j = 0; j < k; ++j) {
         CPM_CUDA_TRY(cudaMemcpyAsync(dx.p, x + (size_t)j * D, D * 8, cudaMemcpyHostToDevice, stream()));
         launch_epass<double, 1>(v, nullptr, -1, dx.p, dt.p, stream());
-        k_lpass<double, 1><<<row_grid(D, 1), BS, 0, stream()>>>(v, m, n, dx.p, dt.p, dy.p);
+        launch_after(k_lpass<double, 1>, row_grid(D, 1), BS, stream(), v, m, n, dx.p, dt.p, dy.p);
         CPM_CUDA_TRY(cudaGetLastError());
         CPM_CUDA_TRY(cudaMemcpyAsync(y + (size_t)j * D, dy.p, D * 8, cudaMemcpyDeviceToHost, stream()));
     }
@@ -2511,7 +2561,7 @@ extern "C" int cpm_explicit_step(cpm_opset_t op, double dt, int32_t k, const dou
     auto v = op->view<double>();
     for (int j = 0; j < k; ++j) {
         CPM_CUDA_TRY(cudaMemcpyAsync(du.p, u + (size_t)j * D, D * 8, cudaMemcpyHostToDevice, stream()));
-        k_lpass<double, 1><<<row_grid(D, 1), BS, 0, stream()>>>(v, 1.0, dt, du.p, du.p, dv.p);
+        launch_after(k_lpass<double, 1>, row_grid(D, 1), BS, stream(), v, 1.0, dt, du.p, du.p, dv.p);
         if (v.n_ident > 0) k_scale_ident<<<nblk(v.n_ident), BS, 0, stream()>>>(v.ident, v.n_ident, 1.0 + dt, du.p, dv.p);
         CPM_CUDA_TRY(cudaGetLastError());
         launch_epass<double, 1>(v, nullptr, -1, dv.p, du.p, stream());
@@ -2546,8 +2596,8 @@ extern "C" int cpm_gray_scott_step(cpm_opset_t op, double dt, double F, double k
     CPM_TRY(dun.alloc(D));
     CPM_TRY(dvn.alloc(D));
     auto w = op->view<double>();
-    k_lpass<double, 1><<<row_grid(D, 1), BS, 0, stream()>>>(w, 1.0, nu_u * dt, du.p, du.p, dun.p);
-    k_lpass<double, 1><<<row_grid(D, 1), BS, 0, stream()>>>(w, 1.0, nu_v * dt, dv.p, dv.p, dvn.p);
+    launch_after(k_lpass<double, 1>, row_grid(D, 1), BS, stream(), w, 1.0, nu_u * dt, du.p, du.p, dun.p);
+    launch_after(k_lpass<double, 1>, row_grid(D, 1), BS, stream(), w, 1.0, nu_v * dt, dv.p, dv.p, dvn.p);
     if (w.n_ident > 0) {
         k_scale_ident<<<nblk(w.n_ident), BS, 0, stream()>>>(w.ident, w.n_ident, 1.0 + nu_u * dt, du.p, dun.p);
         k_scale_ident<<<nblk(w.n_ident), BS, 0, stream()>>>(w.ident, w.n_ident, 1.0 + nu_v * dt, dv.p, dvn.p);
@@ -2575,16 +2625,16 @@ extern "C" int cpm_apply_device(cpm_opset_t op, double m, double n, int32_t kslo
         float *t = (float *)t_dev, *y = (float *)y_dev;
         if (kslots == 1) {
             launch_epass<float, 1>(v, nullptr, -1, x, t, st);
-            k_lpass<float, 1><<<row_grid(D, 1), BS, 0, st>>>(v, (float)m, (float)n, x, t, y);
+            launch_after(k_lpass<float, 1>, row_grid(D, 1), BS, st, v, (float)m, (float)n, x, t, y);
         } else {
             launch_epass<float, 32>(v, nullptr, -1, x, t, st);
             if (lpass4_ok(D, x, t, y))
                 if (v.ov_ptr)
-                    k_lpass4<true><<<row_grid(D, 32), BS, 0, st>>>(v, (float)m, (float)n, x, t, y);
+                    launch_after(k_lpass4<true>, row_grid(D, 32), BS, st, v, (float)m, (float)n, x, t, y);
                 else
-                    k_lpass4<false><<<row_grid(D, 32), BS, 0, st>>>(v, (float)m, (float)n, x, t, y);
+                    launch_after(k_lpass4<false>, row_grid(D, 32), BS, st, v, (float)m, (float)n, x, t, y);
             else
-                k_lpass<float, 32><<<row_grid(D, 32), BS, 0, st>>>(v, (float)m, (float)n, x, t, y);
+                launch_after(k_lpass<float, 32>, row_grid(D, 32), BS, st, v, (float)m, (float)n, x, t, y);
         }
     } else {
         auto v = op->view<double>();
@@ -2592,10 +2642,10 @@ extern "C" int cpm_apply_device(cpm_opset_t op, double m, double n, int32_t kslo
         double *t = (double *)t_dev, *y = (double *)y_dev;
         if (kslots == 1) {
             launch_epass<double, 1>(v, nullptr, -1, x, t, st);
-            k_lpass<double, 1><<<row_grid(D, 1), BS, 0, st>>>(v, m, n, x, t, y);
+            launch_after(k_lpass<double, 1>, row_grid(D, 1), BS, st, v, m, n, x, t, y);
         } else {
             launch_epass<double, 32>(v, nullptr, -1, x, t, st);
-            k_lpass<double, 32><<<row_grid(D, 32), BS, 0, st>>>(v, m, n, x, t, y);
+            launch_after(k_lpass<double, 32>, row_grid(D, 32), BS, st, v, m, n, x, t, y);
         }
     }
     count_launches(1 + (kslots == 32 ? (fp32 ? epass_kernels<float, 32>(op->view<float>(), (const float *)x_dev)
@@ -2758,16 +2808,16 @@ extern "C" int cpm_apply_device_noalloc(cpm_opset_t op, double m, double n, int3
         float *tt = (float *)t, *y = (float *)y_dev;
         if (kslots == 1) {
             launch_epass<float, 1>(v, nullptr, -1, x, tt, st);
-            k_lpass<float, 1><<<row_grid(D, 1), BS, 0, st>>>(v, (float)m, (float)n, x, tt, y);
+            launch_after(k_lpass<float, 1>, row_grid(D, 1), BS, st, v, (float)m, (float)n, x, tt, y);
         } else {
             launch_epass<float, 32>(v, nullptr, -1, x, tt, st);
             if (lpass4_ok(D, x, tt, y))
                 if (v.ov_ptr)
-                    k_lpass4<true><<<row_grid(D, 32), BS, 0, st>>>(v, (float)m, (float)n, x, tt, y);
+                    launch_after(k_lpass4<true>, row_grid(D, 32), BS, st, v, (float)m, (float)n, x, tt, y);
                 else
-                    k_lpass4<false><<<row_grid(D, 32), BS, 0, st>>>(v, (float)m, (float)n, x, tt, y);
+                    launch_after(k_lpass4<false>, row_grid(D, 32), BS, st, v, (float)m, (float)n, x, tt, y);
             else
-                k_lpass<float, 32><<<row_grid(D, 32), BS, 0, st>>>(v, (float)m, (float)n, x, tt, y);
+                launch_after(k_lpass<float, 32>, row_grid(D, 32), BS, st, v, (float)m, (float)n, x, tt, y);
         }
     } else {
         auto v = op->view<double>();
@@ -2775,10 +2825,10 @@ extern "C" int cpm_apply_device_noalloc(cpm_opset_t op, double m, double n, int3
         double *tt = (double *)t, *y = (double *)y_dev;
         if (kslots == 1) {
             launch_epass<double, 1>(v, nullptr, -1, x, tt, st);
-            k_lpass<double, 1><<<row_grid(D, 1), BS, 0, st>>>(v, m, n, x, tt, y);
+            launch_after(k_lpass<double, 1>, row_grid(D, 1), BS, st, v, m, n, x, tt, y);
         } else {
             launch_epass<double, 32>(v, nullptr, -1, x, tt, st);
-            k_lpass<double, 32><<<row_grid(D, 32), BS, 0, st>>>(v, m, n, x, tt, y);
+            launch_after(k_lpass<double, 32>, row_grid(D, 32), BS, st, v, m, n, x, tt, y);
         }
     }
     count_launches(1 + (kslots == 32 ? (fp32 ? epass_kernels<float, 32>(op->view<float>(), (const float *)x_dev)
