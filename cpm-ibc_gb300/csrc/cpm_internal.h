@@ -140,6 +140,7 @@ struct SurfaceParams {
     // mesh (triangles / segments) with a uniform cell grid for candidate search
     const double *verts;     // device, 3*nv
     const int32_t *prims;    // device, 3*np or 2*np
+    const float4 *sph;       // device, np: a sphere around each primitive (centre, radius rounded up)
     int64_t nprims;
     const int32_t *cell_start;  // device, ncell+1
     const int32_t *cell_items;  // device
@@ -180,6 +181,7 @@ __device__ __forceinline__ int node_at(const BrickView &b, int i, int j, int k) 
 struct Mesh {
     DBuf<double> verts;
     DBuf<int32_t> prims, cell_start, cell_items;
+    DBuf<float4> sph;
     int64_t nprims = 0;
     double glo[3] = {0, 0, 0}, gh = 0;
     int gn[3] = {0, 0, 0};
