@@ -683,61 +683,51 @@ __device__ __forceinline__ double e1_row(const OpView<double> &op, int64_t p, ui
     return fx_to_double(fx_dot4(ax, wx), e20);
 }
 
+// one warp's run: the operator's tables of it
+struct E1Run {
+    int4 ch;
+    int ca[E1_GROUPS], cb[E1_GROUPS], r;
+    uint8_t fl;
+    int64_t p;
+};
 template <class T>
-__global__ void __launch_bounds__(E1_T, 7) k_epass1(OpView<T> op, const Slot *sl, int ph, unsigned row_blocks,
-                                                 const T *x, T *t) {
-    __shared__ E1Group<T> sh[E1_T / 32][E1_GROUPS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t c = (int64_t)blockIdx.x * (E1_T / 32) + warp;
-    const bool rows = blockIdx.x < row_blocks && c < op.n_chunk;
-    // the operator's own tables while the previous kernel ends
-    int4 ch = make_int4(0, 0, 0, 0);
-    int ca[E1_GROUPS], cb[E1_GROUPS], r = 0;
-    uint8_t fl = 0;
-    int64_t p = 0;
-    if (rows) {
-        ch = __ldg(op.chunk + c);
-        const int32_t *gc = op.gcols + 64 * (int64_t)ch.x + lane;
+__device__ __forceinline__ void e1_tables(const OpView<T> &op, int64_t c, int lane, E1Run &q) {
+    q.ch = __ldg(op.chunk + c);
+    const int32_t *gc = op.gcols + 64 * (int64_t)q.ch.x + lane;
 #pragma unroll
-        for (int g = 0; g < E1_GROUPS; ++g)
-            if (g < ch.w >> 8) {
-                ca[g] = __ldg(gc + 64 * g);
-                cb[g] = __ldg(gc + 64 * g + 32);
-            }
-        p = ch.y + min(lane, (ch.w & 255) - 1);
-        r = __ldg(op.ord + p);
-        fl = __ldg(op.fl_ord + p) & F_TERMS;
-    }
-    pdl_wait();
-    if (ph >= 0 && sl[0].phase != ph) return;
-    if (blockIdx.x >= row_blocks) {  // identity rows
-        const int64_t q = (int64_t)(blockIdx.x - row_blocks) * E1_T + threadIdx.x;
-        if (q < op.n_ident) {
-            const int ri = op.ident[q];
-            t[ri] = x[ri];
+    for (int g = 0; g < E1_GROUPS; ++g)
+        if (g < q.ch.w >> 8) {
+            q.ca[g] = __ldg(gc + 64 * g);
+            q.cb[g] = __ldg(gc + 64 * g + 32);
         }
-        return;
-    }
-    if (!rows) return;
-    const int ng = ch.w >> 8, nr = ch.w & 255;
+    q.p = q.ch.y + min(lane, (q.ch.w & 255) - 1);
+    q.r = __ldg(op.ord + q.p);
+    q.fl = __ldg(op.fl_ord + q.p) & F_TERMS;
+}
+// and its rows of t
+template <class T>
+__device__ __forceinline__ void e1_run(const OpView<T> &op, const E1Run &q, int lane, E1Group<T> (&sh)[E1_GROUPS], const T *x,
+                                       T *t) {
+    const int ng = q.ch.w >> 8, nr = q.ch.w & 255;
     T xa[E1_GROUPS], xb[E1_GROUPS];
 #pragma unroll
     for (int g = 0; g < E1_GROUPS; ++g)
         if (g < ng) {
-            xa[g] = x[ca[g]];
-            xb[g] = x[cb[g]];
+            xa[g] = x[q.ca[g]];
+            xb[g] = x[q.cb[g]];
         }
-    const int mine = __popc((uint32_t)ch.z & (0xffffffffu >> (31 - lane))) - 1;  // the row's group
+    const int mine = __popc((uint32_t)q.ch.z & (0xffffffffu >> (31 - lane))) - 1;  // the row's group
     uint32_t e20 = FX_EMIN;  // exponent field of the row's group
     bool zero = false;       // the warp's groups of smallest exponent hold zeros only
+    __syncwarp();
     if constexpr (sizeof(T) == 8) {
 #pragma unroll
         for (int g = 0; g < E1_GROUPS; ++g)
             if (g < ng) {
                 const uint32_t e = __reduce_max_sync(FULL, max(exp_field(xa[g]), exp_field(xb[g])));
                 if (mine == g) e20 = e;
-                sh[warp][g].x[lane] = fx_from_double(xa[g], e);
-                sh[warp][g].x[lane + 32] = fx_from_double(xb[g], e);
+                sh[g].x[lane] = fx_from_double(xa[g], e);
+                sh[g].x[lane + 32] = fx_from_double(xb[g], e);
             }
         if (__any_sync(FULL, e20 == 0)) {
             bool nz = false;
@@ -751,17 +741,39 @@ __global__ void __launch_bounds__(E1_T, 7) k_epass1(OpView<T> op, const Slot *sl
 #pragma unroll
         for (int g = 0; g < E1_GROUPS; ++g)
             if (g < ng) {
-                sh[warp][g].x[lane] = xa[g];
-                sh[warp][g].x[lane + 32] = xb[g];
+                sh[g].x[lane] = xa[g];
+                sh[g].x[lane + 32] = xb[g];
             }
     }
     __syncwarp();
-    T acc = e1_row(op, p, e20, sh[warp][mine]);
+    T acc = e1_row(op, q.p, e20, sh[mine]);
     if constexpr (sizeof(T) == 8)
-        if (fx_out(e20)) acc = zero ? 0.0 : e_row_fp64<1>(op.w_ord + 12 * p, op.gcols + 64 * (int64_t)(ch.x + mine), 0, x);
+        if (fx_out(e20)) acc = zero ? 0.0 : e_row_fp64<1>(op.w_ord + 12 * q.p, op.gcols + 64 * (int64_t)(q.ch.x + mine), 0, x);
     if (lane < nr) {
-        if (fl) acc = e_row_terms<T, 1>(op, fl, r, 0, acc, x);
-        t[r] = acc;
+        if (q.fl) acc = e_row_terms<T, 1>(op, q.fl, q.r, 0, acc, x);
+        t[q.r] = acc;
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(E1_T, 7) k_epass1(OpView<T> op, const Slot *sl, int ph, unsigned row_blocks,
+                                                 const T *x, T *t) {
+    __shared__ E1Group<T> sh[E1_T / 32][E1_GROUPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * (E1_T / 32) + warp;
+    const bool rows = blockIdx.x < row_blocks && c < op.n_chunk;
+    E1Run q;
+    if (rows) e1_tables(op, c, lane, q);  // while the previous kernel ends
+    pdl_wait();
+    if (ph >= 0 && sl[0].phase != ph) return;
+    if (rows) {
+        e1_run(op, q, lane, sh[warp], x, t);
+    } else if (blockIdx.x >= row_blocks) {  // identity rows
+        const int64_t k = (int64_t)(blockIdx.x - row_blocks) * E1_T + threadIdx.x;
+        if (k < op.n_ident) {
+            const int r = op.ident[k];
+            t[r] = x[r];
+        }
     }
 }
 
@@ -1469,6 +1481,176 @@ __global__ void __launch_bounds__(BS, 4) k_restart(OpView<T> op, Slot *sl, T m, 
     }
 }
 
+// ---- BiCGStab for one FP64 vector in one kernel.  At these sizes (11 to 300
+// thousand rows) an iteration is seven kernels of 3 to 15 us, and with Jacobi
+// sweeps thousands of 5 us, of which starting, reading the slot's phase and
+// draining take more than half; here the blocks of a cooperative launch stay and
+// meet at a barrier (1.3 us) wherever rows of other blocks are read, the
+// operator's tables of a warp's first run stay in registers, and a solve stops at
+// the iteration that converges instead of the end of a graph.
+struct Plain1 {
+    OpView<double> op;
+    Slot *sl;
+    SolveParams P;
+    double m, n, ys;
+    const double *pinv;  // null: no preconditioner
+    double *x, *r, *r0, *p, *v, *s, *t, *y, *z, *te;
+    double *partial;     // the blocks' two sums, one place for each of an iteration's three reductions
+    unsigned int *bar;   // arrivals, zero at launch; bar[1]: a wait ran out
+    int iters;           // iterations at most
+};
+
+// Barrier over the grid (a cooperative launch: every block is resident): 1.2 us
+// with 152 blocks, 1.5 with 304.  (A word per block that all blocks read took 5 us
+// and more: the readers hold up the writes.)  A wait that runs out, some seconds,
+// sets bar[1] and every block leaves: false.
+constexpr int PLAIN1_POLLS = 1 << 22;
+__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned &target) {
+    __shared__ bool met;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        target += gridDim.x;
+        // releases the block's writes, ordered before by the __syncthreads
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        bool ok = false;
+        for (int i = 0; i < PLAIN1_POLLS; ++i) {
+            unsigned now;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
+            if ((int)(now - target) >= 0) {
+                ok = true;
+                break;
+            }
+            if ((i & 1023) == 1023 && *(volatile unsigned int *)(bar + 1)) break;
+        }
+        if (!ok) atomicExch(bar + 1, 1u);
+        met = ok;
+    }
+    __syncthreads();
+    return met;
+}
+
+constexpr int PLAIN1_BPS = 2;  // blocks per SM at most
+__global__ void __launch_bounds__(BS, PLAIN1_BPS) k_plain1(Plain1 a) {
+    constexpr int K = 1;
+    __shared__ E1Group<double> eg[BS / 32][E1_GROUPS];
+    __shared__ Slot S;
+    __shared__ double sh[2][BS];
+    const OpView<double> &op = a.op;
+    const int64_t D = op.D;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    GRID_LOOP
+    const int64_t warps = (int64_t)gridDim.x * (BS / 32), c0 = (int64_t)blockIdx.x + (int64_t)warp * gridDim.x;
+    E1Run run;
+    if (c0 < op.n_chunk) e1_tables(op, c0, lane, run);
+    if (tid == 0) S = a.sl[0];
+    unsigned target = 0;
+    bool ok = true;
+    __syncthreads();
+
+    // sums over the grid, in thread 0 of every block (the same bits in each)
+    auto reduce = [&](double (&v)[2], double *partial) {
+        __syncthreads();
+        block_tree<2>(v, sh);
+        if (tid == 0) {
+            partial[2 * blockIdx.x] = v[0];
+            partial[2 * blockIdx.x + 1] = v[1];
+        }
+        ok = grid_barrier(a.bar, target);
+        v[0] = v[1] = 0.0;
+        for (unsigned b = tid; b < gridDim.x; b += BS) {
+            v[0] += __ldcg(partial + 2 * b);
+            v[1] += __ldcg(partial + 2 * b + 1);
+        }
+        block_tree<2>(v, sh);
+    };
+
+    for (int it = 0; it < a.iters && S.phase == PH_ITER; ++it) {
+        // p and y, v = A y, alpha; then s and z, t = A z, omega
+        for (int half = 0; half < 2; ++half) {
+            const double c1 = half ? S.alpha : S.omega, beta = S.beta;
+            const double *in = half ? a.s : a.p;
+            double *y = half ? a.z : a.y, *o = half ? a.t : a.v;
+            for (int64_t q = r0i; q < D; q += rstride) {
+                double e;
+                if (half) {  // s = r - alpha v
+                    e = fma(-c1, a.v[q], a.r[q]);
+                    a.s[q] = e;
+                } else {     // p = (p - w v) beta + r
+                    e = fma(fma(-c1, a.v[q], a.p[q]), beta, a.r[q]);
+                    a.p[q] = e;
+                }
+                y[q] = a.pinv ? a.ys * (e * a.pinv[q]) : e;  // M^-1, or the first Jacobi sweep
+            }
+            double dot[2] = {0.0, 0.0};
+            const int passes = a.P.precond == 2 ? a.P.sweeps : 1;
+            for (int j = 1; j <= passes; ++j) {
+                // te = E~ y: every block's rows of y first, every row of te before it is read
+                if (!(ok = grid_barrier(a.bar, target))) return;
+                for (int64_t c = c0; c < op.n_chunk; c += warps) {
+                    if (c != c0) e1_tables(op, c, lane, run);
+                    e1_run(op, run, lane, eg[warp], (const double *)y, a.te);
+                }
+                if (c0 + warps < op.n_chunk) e1_tables(op, c0, lane, run);
+                for (int64_t k = (int64_t)blockIdx.x * BS + tid; k < op.n_ident; k += (int64_t)gridDim.x * BS) {
+                    const int r = op.ident[k];
+                    a.te[r] = y[r];
+                }
+                if (!(ok = grid_barrier(a.bar, target))) return;
+                const bool last = j == passes;
+                constexpr int UN = 2;
+                ROWS_UNR_N(D, UN) {
+                    ROWS_OF_TRIP_N(rr, UN)
+                    double ay[UN], w[UN], dv[UN];
+#pragma unroll
+                    for (int u = 0; u < UN; ++u) {
+                        w[u] = dv[u] = 0.0;
+                        if (rr[u] < D) {
+                            w[u] = (last && !half) ? a.r0[rr[u]] : in[rr[u]];
+                            if (!last) dv[u] = a.pinv[rr[u]];
+                        }
+                    }
+                    l_rows<double, 1, UN>(op, rr, s, a.m, a.n, (const double *)y, a.te, true, ay);
+#pragma unroll
+                    for (int u = 0; u < UN; ++u)
+                        if (rr[u] < D) {
+                            if (last) {
+                                o[rr[u]] = ay[u];
+                                dot[1] += ay[u] * w[u];
+                                if (half) dot[0] += ay[u] * ay[u];
+                            } else {  // a further Jacobi sweep on A y = in
+                                y[rr[u]] += JACOBI_OMEGA * ((w[u] - ay[u]) * dv[u]);
+                            }
+                        }
+                }
+            }
+            reduce(dot, a.partial + 2 * (size_t)gridDim.x * half);
+            if (!ok) return;
+            if (tid == 0) {
+                if (half)
+                    omega_update(S, dot[0], dot[1]);
+                else
+                    alpha_update<double>(S, dot[1]);
+            }
+            __syncthreads();
+        }
+        // x += alpha y + w z ; r = s - w t
+        const double al = S.alpha, w = S.omega;
+        double dot[2] = {0.0, 0.0};
+        for (int64_t q = r0i; q < D; q += rstride) {
+            a.x[q] = fma(w, a.z[q], fma(al, a.y[q], a.x[q]));
+            const double ri = fma(-w, a.t[q], a.s[q]);
+            a.r[q] = ri;
+            dot[0] += ri * ri;
+            dot[1] += a.r0[q] * ri;
+        }
+        reduce(dot, a.partial + 4 * (size_t)gridDim.x);
+        if (!ok) return;
+        if (tid == 0) xr_update(S, a.P, dot[0], dot[1]);
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && tid == 0) a.sl[0] = S;
+}
+
 // reliable updates run for all slots at once every few iterations, so one FP64
 // apply serves every slot that needs it: a slot joins when its FP32 residual has
 // fallen by delta since its last update (Sleijpen & van der Vorst's criterion),
@@ -1714,6 +1896,7 @@ struct cpm_solver_s {
     int G = 1;
     DBuf<Slot> slots;
     PinnedArray<Slot> h_slots;  // pinned: the slot read-back after a graph does not block the host
+    PinnedArray<unsigned int> h_bar;
     DBuf<double> partial;
     DBuf<unsigned int> counter;
     // FP64 Krylov vectors (plain path) and FP64 refinement state (mixed path)
@@ -1725,6 +1908,10 @@ struct cpm_solver_s {
     // captured iteration graphs (kernel arguments are fixed pointers; per-solve
     // parameters live in device memory, so a graph is reused while they match)
     cudaGraphExec_t g_plain = nullptr, g_mixed = nullptr;
+    // k_plain1's grid (0: this solver iterates by graphs), partial sums and barrier
+    int plain1_G = 0;
+    DBuf<double> plain1_partial;
+    DBuf<unsigned int> plain1_bar;
     SolveParams gp_plain{}, gp_mixed{};
     int chunk = 16;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -1795,6 +1982,32 @@ static void plain_iteration(cpm_solver_s *s, const SolveParams &P) {
                                                   s->counter.p);
     launch_after(k_update_xr<double, K>, s->G, BS, st, D, sl, P, s->dy.p, s->dz.p, s->ds.p, s->dt.p, s->dr0.p, s->x64.p, s->dr.p,
                                                 s->partial.p, s->counter.p);
+}
+
+// rows up to which one kernel iterates (216 thousand: 65 us an iteration, 68 by
+// the graph's kernels; these are long enough above, and hold more warps)
+constexpr int64_t PLAIN1_MAX_D = 250000;
+// one launch of k_plain1: iterations until the slot leaves PH_ITER, at most `iters`
+static int plain1_blocks(const cpm_solver_s *s) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_plain1, BS, 0) != cudaSuccess || per_sm < 1) return 0;
+    // one block per SM as long as its eight warps cover the runs (22 thousand rows: 30.8
+    // us an iteration, 35.5 with two blocks), else two (42 thousand: 8.6 us a sweep, 11.0
+    // with one).  Small systems spread over the SMs rather than fill eight warps.
+    const int64_t sms = sm_count(), runs = std::max<int64_t>(1, s->op->n_chunk);
+    const int64_t most = runs <= sms * (BS / 32) ? sms : sms * std::min(per_sm, PLAIN1_BPS);
+    return (int)std::min<int64_t>(most, std::max<int64_t>(runs, (s->D + BS - 1) / BS));
+}
+static int plain1_launch(cpm_solver_s *s, const SolveParams &P, int iters) {
+    cudaStream_t st = stream();
+    Plain1 a{s->op->view<double>(), s->slots.p, P, s->m, s->n, P.precond == 2 ? JACOBI_OMEGA : 1.0,
+             P.precond == 0 ? nullptr : s->pinv64.p, s->x64.p, s->dr.p, s->dr0.p, s->dp.p, s->dv.p, s->ds.p, s->dt.p, s->dy.p,
+             s->dz.p, s->te64.p, s->plain1_partial.p, s->plain1_bar.p, iters};
+    CPM_CUDA_TRY(cudaMemsetAsync(s->plain1_bar.p, 0, 2 * sizeof(unsigned int), st));
+    void *args[] = {&a};
+    CPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_plain1, dim3(s->plain1_G), dim3(BS), args, 0, st));
+    count_launches(1);
+    return 0;
 }
 
 template <int K>
@@ -1903,6 +2116,9 @@ static int parse_params(const cpm_solve_opts *o, SolveParams &P) {
     return 0;
 }
 
+// iterations per launch of k_plain1 (with Jacobi sweeps: some ten thousand barriers)
+static inline int plain1_iters(const SolveParams &P) { return P.precond == 2 ? std::max(1, 4000 / P.sweeps) : 128; }
+
 // iterations per captured graph
 // (Jacobi-preconditioned solves: one iteration, already thousands of launches;
 // mixed: 32 iterations, so that the reliable-update period can reach 32)
@@ -1999,16 +2215,23 @@ static int solve_pass(cpm_solver_s *s, const SolveParams &P, const std::vector<c
     }
     CPM_CUDA_TRY(cudaGetLastError());
     cudaGraphExec_t gexec = nullptr;
-    CPM_TRY(prepare_graph<K>(s, P, &gexec));
-    const int chunk = graph_chunk(s, P);
+    const bool one_kernel = K == 1 && !P.mixed && s->plain1_G > 0;
+    if (!one_kernel) CPM_TRY(prepare_graph<K>(s, P, &gexec));
+    const int chunk = one_kernel ? plain1_iters(P) : graph_chunk(s, P);
     const int64_t max_chunks = (int64_t)P.max_iters / chunk + 2 * P.max_refine + 4;
     const long long per_graph = graph_launches(s, P);
     bool done = false;
     for (int64_t c = 0; c < max_chunks && !done; ++c) {
-        CPM_CUDA_TRY(cudaGraphLaunch(gexec, st));
-        count_launches(per_graph);
+        if (one_kernel) {
+            CPM_TRY(plain1_launch(s, P, chunk));
+            CPM_CUDA_TRY(cudaMemcpyAsync(&s->h_bar[0], s->plain1_bar.p + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+        } else {
+            CPM_CUDA_TRY(cudaGraphLaunch(gexec, st));
+            count_launches(per_graph);
+        }
         CPM_CUDA_TRY(cudaMemcpyAsync(s->h_slots.data(), s->slots.p, sizeof(Slot) * K, cudaMemcpyDeviceToHost, st));
         CPM_CUDA_TRY(cudaStreamSynchronize(st));
+        if (one_kernel && s->h_bar[0]) return fail(CPM_ERR_TIMEOUT, "solve: a grid barrier ran out");
         done = true;
         bool restart = false;
         for (int j = 0; j < K; ++j) {
@@ -2135,6 +2358,12 @@ extern "C" int cpm_solver_create(cpm_opset_t op, double m, double n, int32_t ksl
         return bail(rc);
     k_pinv<double><<<nblk(s->D), BS, 0, stream()>>>(op->view<double>(), m, n, s->pinv64.p);
     if (cudaGetLastError() != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "pinv kernel"));
+    if (s->K == 1 && s->D <= PLAIN1_MAX_D) {
+        s->plain1_G = plain1_blocks(s);
+        if ((rc = s->plain1_partial.alloc(6 * (size_t)std::max(1, s->plain1_G))) || (rc = s->plain1_bar.alloc(2)) ||
+            (rc = s->h_bar.alloc(1)))
+            return bail(rc);
+    }
     cudaEventCreate(&s->e0);
     cudaEventCreate(&s->e1);
     if (cudaStreamSynchronize(s->own) != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "solver_create"));
