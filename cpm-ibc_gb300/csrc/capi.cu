@@ -1,5 +1,6 @@
 // Library-wide state of the C-ABI: per-thread error strings, the library
 // stream, device queries.
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -31,6 +32,49 @@ cudaStream_t library_stream() {
 static thread_local cudaStream_t g_scope = nullptr;
 
 cudaStream_t stream() { return g_scope ? g_scope : library_stream(); }
+
+Scratch *&Scratch::current() {
+    static thread_local Scratch *s = nullptr;
+    return s;
+}
+void *Scratch::take(size_t bytes) {
+    bytes = (bytes + 255) & ~(size_t)255;
+    while (at < chunks.size() && used + bytes > chunks[at].bytes) {
+        ++at;
+        used = 0;
+    }
+    if (at == chunks.size()) {
+        Chunk c{nullptr, std::max(bytes, chunks.empty() ? (size_t)(16 << 20) : 2 * chunks.back().bytes)};
+        if (cudaMalloc((void **)&c.p, c.bytes) != cudaSuccess) {
+            cudaGetLastError();
+            c.bytes = bytes;  // doubling may be what does not fit
+            if (cudaMalloc((void **)&c.p, c.bytes) != cudaSuccess) return nullptr;
+        }
+        chunks.push_back(c);
+        used = 0;
+    }
+    void *p = chunks[at].p + used;
+    used += bytes;
+    return p;
+}
+Scratch::~Scratch() {
+    for (Chunk &c : chunks) cudaFree(c.p);
+}
+ScratchScope::ScratchScope() {
+    Scratch *&cur = Scratch::current();
+    if (!cur) cur = own = new Scratch();
+    at = cur->at;
+    used = cur->used;
+}
+ScratchScope::~ScratchScope() {
+    Scratch *&cur = Scratch::current();
+    cur->at = at;
+    cur->used = used;
+    if (own) {
+        cur = nullptr;
+        delete own;
+    }
+}
 
 StreamScope::StreamScope(cudaStream_t s) : prev(g_scope) { g_scope = s; }
 StreamScope::~StreamScope() { g_scope = prev; }

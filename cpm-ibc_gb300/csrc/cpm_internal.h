@@ -101,6 +101,59 @@ struct DBuf {
     }
 };
 
+// Device memory for the temporaries of one build or query.  cudaMalloc and
+// cudaFree take 95 us a buffer on this machine and a set-up has some 200 of them,
+// so the outermost ScratchScope of a call takes a few chunks, TBufs are places in
+// them, and all is given back when it ends.  A scope inside another one gives its
+// places back at its end; what used them and what gets them next are on one
+// stream.  Per thread; a TBuf outside any scope owns its memory.
+struct Scratch {
+    struct Chunk {
+        char *p;
+        size_t bytes;
+    };
+    std::vector<Chunk> chunks;
+    size_t at = 0, used = 0;  // the chunk in use and its used bytes
+    static Scratch *&current();
+    void *take(size_t bytes);  // nullptr: out of memory
+    ~Scratch();
+};
+struct ScratchScope {
+    ScratchScope();
+    ~ScratchScope();
+    ScratchScope(const ScratchScope &) = delete;
+    ScratchScope &operator=(const ScratchScope &) = delete;
+    Scratch *own = nullptr;  // the outermost scope's
+    size_t at = 0, used = 0;
+};
+template <class T>
+struct TBuf : DBuf<T> {
+    bool placed = false;
+    TBuf() = default;
+    ~TBuf() {
+        if (placed) this->p = nullptr;
+    }
+    int alloc(size_t count) {
+        Scratch *s = Scratch::current();
+        if (placed) this->p = nullptr;
+        placed = false;
+        if (!s) return DBuf<T>::alloc(count);
+        this->release();
+        if (count == 0) count = 1;
+        this->p = (T *)s->take(count * sizeof(T));
+        if (!this->p) return fail(CPM_ERR_OOM, "scratch memory");
+        placed = true;
+        this->n = count;
+        return 0;
+    }
+    int upload(const T *h, size_t count) {
+        CPM_TRY(alloc(count));
+        CPM_CUDA_TRY(cudaMemcpyAsync(this->p, h, count * sizeof(T), cudaMemcpyHostToDevice, stream()));
+        return 0;
+    }
+    int upload(const std::vector<T> &h) { return upload(h.data(), h.size()); }
+};
+
 // Host array in page-locked memory.  A device-to-host cudaMemcpyAsync into
 // pageable memory returns only once the copy (and so all earlier work on its
 // stream) is done; into a PinnedArray it is queued like any other stream work.

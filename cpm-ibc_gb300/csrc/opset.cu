@@ -207,13 +207,14 @@ struct QueryRows {  // base points + weights of query points (computed on the de
 };
 
 static int query_weights(const cpm_tube_s *t, const std::vector<double> &pts, QueryRows &out) {
+    ScratchScope scratch;
     int64_t n = (int64_t)pts.size() / 3;
     out.base.clear();
     out.w.clear();
     if (n == 0) return 0;
-    DBuf<double> dp, dw;
-    DBuf<uint32_t> db;
-    DBuf<int32_t> err;
+    TBuf<double> dp, dw;
+    TBuf<uint32_t> db;
+    TBuf<int32_t> err;
     CPM_TRY(dp.upload(pts));
     CPM_TRY(db.alloc(n));
     CPM_TRY(dw.alloc(12 * n));
@@ -452,14 +453,15 @@ __global__ void k_tag_frames(BrickView bv, int64_t nt, const uint32_t *__restric
 // the frame directions of an IBC's tagging subset, computed on the device from
 // the tube's unoriented normals (3 N, device)
 static int tag_frames_dev(cpm_tube_s *t, IBCData &ib, const double *normals_dev) {
+    ScratchScope scratch;
     const int64_t nt = (int64_t)ib.tag_set.size();
     ib.tag_dir.assign(3 * nt, 0.0);
     ib.tag_binormal.assign(3 * nt, 0.0);
     if (nt == 0) return 0;
     std::vector<int32_t> set(ib.tag_set.begin(), ib.tag_set.end()), sub(ib.tag_sub.begin(), ib.tag_sub.end());
-    DBuf<int32_t> dset, dsub, derr;
-    DBuf<double> dcpc, dcd, dg, ddir, dbn, dw;
-    DBuf<uint32_t> db;
+    TBuf<int32_t> dset, dsub, derr;
+    TBuf<double> dcpc, dcd, dg, ddir, dbn, dw;
+    TBuf<uint32_t> db;
     CPM_TRY(dset.upload(set));
     CPM_TRY(dsub.upload(sub));
     CPM_TRY(dcpc.upload(ib.tag_cpc));
@@ -720,8 +722,9 @@ __global__ void k_count_below(int64_t n, const double *__restrict__ v, double li
 }
 
 static int build_ibc_data(cpm_tube_s *t, const HostTube &ht, const cpm_surface_desc &desc, const double *normals_dev,
-                          const DBuf<double> &xdev, const CpTable *cpt, const CpTable *surf_cpt,
+                          const TBuf<double> &xdev, const CpTable *cpt, const CpTable *surf_cpt,
                           IBCData &ib) {
+    ScratchScope scratch;
     const int64_t N = ht.N;
     const double r = ht.radius;
     ib.desc = desc;
@@ -732,7 +735,7 @@ static int build_ibc_data(cpm_tube_s *t, const HostTube &ht, const cpm_surface_d
     CPM_TRY(surface_init(s, &desc, r));
     std::vector<double> verts;
     if (desc.kind == CPM_TRIANGULATION || desc.kind == CPM_POLYLINE) verts.assign(desc.verts, desc.verts + 3 * desc.nverts);
-    DBuf<double> dcp, dd;
+    TBuf<double> dcp, dd;
     CPM_TRY(dcp.alloc(3 * N));
     CPM_TRY(dd.alloc(N));
     CPM_TRY(closest_points_dev(s.params(), N, xdev.p, dcp.p, dd.p, 2.0 * r * (1.0 + 1e-12)));
@@ -765,16 +768,16 @@ static int build_ibc_data(cpm_tube_s *t, const HostTube &ht, const cpm_surface_d
     if (start < 0) return fail(CPM_ERR_INVALID_ARG, "IBC start point is not near the tube");
     {
         // the walk on the device (k_tag_walk), sized by the nodes within 2r
-        DBuf<unsigned long long> dcnt;
+        TBuf<unsigned long long> dcnt;
         CPM_TRY(dcnt.alloc(1));
         CPM_TRY(dcnt.zero());
         k_count_below<<<(unsigned)((N + 255) / 256), 256, 0, stream()>>>(N, dd.p, 2.0 * r, dcnt.p);
         std::vector<unsigned long long> hc;
         CPM_TRY(dcnt.download(hc, 1));
         const int32_t cap = (int32_t)hc[0] + 1;
-        DBuf<uint8_t> vis;
-        DBuf<int32_t> kmin, f0, f1, dset, dn;
-        DBuf<int> derr;
+        TBuf<uint8_t> vis;
+        TBuf<int32_t> kmin, f0, f1, dset, dn;
+        TBuf<int> derr;
         CPM_TRY(vis.alloc(N));
         CPM_TRY(vis.zero());
         CPM_TRY(kmin.alloc(N));
@@ -797,7 +800,7 @@ static int build_ibc_data(cpm_tube_s *t, const HostTube &ht, const cpm_surface_d
         ib.tag_set.assign(hs.begin(), hs.end());
         ib.tag_sub.assign(N, -1);
         for (int64_t i = 0; i < ntw; ++i) ib.tag_sub[hs[i]] = i;
-        DBuf<double> dtc, dtd;
+        TBuf<double> dtc, dtd;
         CPM_TRY(dtc.alloc(3 * std::max<int64_t>(1, ntw)));
         CPM_TRY(dtd.alloc(std::max<int64_t>(1, ntw)));
         if (ntw > 0) {
@@ -844,7 +847,7 @@ static int build_ibc_data(cpm_tube_s *t, const HostTube &ht, const cpm_surface_d
             }
         if (!ends.empty()) {
             const int64_t ne = (int64_t)ends.size();
-            DBuf<double> dp, dcs, dds, dcc, ddc;
+            TBuf<double> dp, dcs, dds, dcc, ddc;
             CPM_TRY(dp.upload(proj));
             CPM_TRY(dcs.alloc(3 * ne));
             CPM_TRY(dds.alloc(ne));
@@ -920,7 +923,7 @@ static int build_ibc_data(cpm_tube_s *t, const HostTube &ht, const cpm_surface_d
         }
         if (desc.has_point_on_side1) {
             const double *ps = desc.point_on_side1;
-            DBuf<double> dps, dcpc, ddc;
+            TBuf<double> dps, dcpc, ddc;
             CPM_TRY(dps.upload(ps, 3));
             CPM_TRY(dcpc.alloc(3));
             CPM_TRY(ddc.alloc(1));
@@ -963,7 +966,7 @@ static int build_ibc_data(cpm_tube_s *t, const HostTube &ht, const cpm_surface_d
             ht.x(ib.dof_set[i], x);
             for (int k = 0; k < 3; ++k) proj[3 * i + k] = 2.0 * ib.dof_cp[3 * i + k] - x[k];
         }
-        DBuf<double> dp, dc, ddist;
+        TBuf<double> dp, dc, ddist;
         CPM_TRY(dp.upload(proj));
         CPM_TRY(dc.alloc(3 * nd));
         CPM_TRY(ddist.alloc(nd));
@@ -1187,9 +1190,10 @@ static int make_float_copies(cpm_opset_s *o) {
 
 // Whole-tube Jcp normals (K7) on the plain (IBC-free) operator rows.
 static int tube_normals(cpm_opset_s *base, std::vector<double> &normals) {
+    ScratchScope scratch;
     cpm_tube_s *t = base->tube;
     const int64_t N = t->N;
-    DBuf<double> g, J, nrm;
+    TBuf<double> g, J, nrm;
     CPM_TRY(g.alloc(9 * N));
     CPM_TRY(J.alloc(9 * N));
     CPM_TRY(nrm.alloc(3 * N));
@@ -1222,12 +1226,12 @@ static int build_ibc(cpm_opset_s *o, int n_ibc, const cpm_surface_desc *descs, c
         CPM_TRY(tube_normals(o, normals));
         CPM_TRY(o->normals.upload(normals));
     }
-    DBuf<double> dnx;
+    TBuf<double> dnx;
     if (need_xn) {
         normals_x = unoriented_normals(ht);
         CPM_TRY(dnx.upload(normals_x));
     }
-    DBuf<double> xdev;
+    TBuf<double> xdev;
     CPM_TRY(xdev.alloc(3 * N));
     k_node_coords<<<(unsigned)((N + 255) / 256), 256, 0, stream()>>>(N, t->key.p, t->g.xstart, t->g.dx, xdev.p);
     CPM_CUDA_TRY(cudaGetLastError());
@@ -1311,9 +1315,9 @@ static int build_ibc(cpm_opset_s *o, int n_ibc, const cpm_surface_desc *descs, c
     // on the device (k_tube_moves): masks and counts, then the targets at scanned offsets
     int64_t nmoved = 0;
     // every IBC's tagging on the device, for the TagStencils kernels
-    std::vector<DBuf<int32_t>> d_tag_sub(n_ibc), d_dof_sub(n_ibc);
-    std::vector<DBuf<uint8_t>> d_tag_bdy(n_ibc);
-    std::vector<DBuf<double>> d_tag_dir(n_ibc);
+    std::vector<TBuf<int32_t>> d_tag_sub(n_ibc), d_dof_sub(n_ibc);
+    std::vector<TBuf<uint8_t>> d_tag_bdy(n_ibc);
+    std::vector<TBuf<double>> d_tag_dir(n_ibc);
     std::vector<IbcTagDev> hib(n_ibc);
     for (int c = 0; c < n_ibc; ++c) {
         const IBCData &ib = ibs[c];
@@ -1332,11 +1336,11 @@ static int build_ibc(cpm_opset_s *o, int n_ibc, const cpm_surface_desc *descs, c
     std::vector<int32_t> ov_ptr{0}, ov_col, ov_s;
     std::vector<double> ov_w;
     if (n_ibc > 0) {
-        DBuf<IbcTagDev> d_ibs;
+        TBuf<IbcTagDev> d_ibs;
         CPM_TRY(d_ibs.upload(hib));
-        DBuf<uint64_t> d_em;
-        DBuf<uint8_t> d_lm;
-        DBuf<int32_t> d_cnt, d_xcnt, d_off, d_moved, d_xoff, d_xcol, d_xsd;
+        TBuf<uint64_t> d_em;
+        TBuf<uint8_t> d_lm;
+        TBuf<int32_t> d_cnt, d_xcnt, d_off, d_moved, d_xoff, d_xcol, d_xsd;
         CPM_TRY(d_em.alloc(N));
         CPM_TRY(d_lm.alloc(N));
         CPM_TRY(d_cnt.alloc(N));
@@ -1416,10 +1420,10 @@ static int build_ibc(cpm_opset_s *o, int n_ibc, const cpm_surface_desc *descs, c
         std::vector<int32_t> dcnt, dlc, dmoved;
         if (nd > 0) {
             std::vector<int32_t> dset(ib.dof_set.begin(), ib.dof_set.end());
-            DBuf<int32_t> d_set, d_cnt, d_lc, d_off, d_mv;
-            DBuf<uint32_t> d_base;
-            DBuf<double> d_dir;
-            DBuf<uint64_t> d_em;
+            TBuf<int32_t> d_set, d_cnt, d_lc, d_off, d_mv;
+            TBuf<uint32_t> d_base;
+            TBuf<double> d_dir;
+            TBuf<uint64_t> d_em;
             CPM_TRY(d_set.upload(dset));
             CPM_TRY(d_base.upload(ib.dof_rows.base));
             CPM_TRY(d_dir.upload(ib.dof_dir));
@@ -1657,7 +1661,7 @@ static int build_schedule(cpm_opset_s *o) {
     k_build_nbr6<<<(unsigned)((N + 255) / 256), 256, 0, stream()>>>(o->view<double>(), o->nbr6.p);
     CPM_CUDA_TRY(cudaGetLastError());
     if (D > N) {
-        DBuf<int> err;
+        TBuf<int> err;
         CPM_TRY(err.alloc(1));
         CPM_TRY(err.zero());
         k_build_nbr6_ibc<<<(unsigned)((D - N + 255) / 256), 256, 0, stream()>>>(o->view<double>(), o->nbr6.p, err.p);
@@ -1776,6 +1780,7 @@ using namespace cpm;
 static int opset_create(cpm_tube_t t, int32_t n_ibc, const cpm_surface_desc *ibcs, const CpOverrides *ovr, cpm_opset_t *out) {
     if (!t || !out || n_ibc < 0 || (n_ibc > 0 && !ibcs)) return fail(CPM_ERR_INVALID_ARG, "invalid arguments");
     *out = nullptr;
+    ScratchScope scratch;
     cpm_opset_s *o = new cpm_opset_s();
     o->tube = t;
     int rc = build_base(o);
@@ -1822,7 +1827,7 @@ static int build_point_batch(cpm_opset_s *o, int n_src, const double *sources, P
     std::vector<double> normals;
     CPM_TRY(tube_normals(o, normals));
     CPM_TRY(o->normals.upload(normals));
-    DBuf<double> xdev;
+    TBuf<double> xdev;
     CPM_TRY(xdev.alloc(3 * N));
     k_node_coords<<<(unsigned)((N + 255) / 256), 256, 0, stream()>>>(N, t->key.p, t->g.xstart, t->g.dx, xdev.p);
     CPM_CUDA_TRY(cudaGetLastError());
@@ -1929,6 +1934,7 @@ static int build_point_batch(cpm_opset_s *o, int n_src, const double *sources, P
 int opset_create_point_batch(cpm_tube_s *t, int n_src, const double *sources, cpm_opset_s **out, PointBatchInfo &info) {
     if (!t || !out || n_src < 1 || n_src > 32 || !sources) return fail(CPM_ERR_INVALID_ARG, "point batch: 1 to 32 sources");
     *out = nullptr;
+    ScratchScope scratch;
     cpm_opset_s *o = new cpm_opset_s();
     o->tube = t;
     int rc = build_base(o);
@@ -1951,6 +1957,7 @@ int opset_create_point_batch(cpm_tube_s *t, int n_src, const double *sources, cp
 extern "C" int cpm_opset_create_identity(cpm_tube_t t, int64_t n_rows, const int64_t *rows, cpm_opset_t *out) {
     if (!t || !out || n_rows < 0 || (n_rows > 0 && !rows)) return fail(CPM_ERR_INVALID_ARG, "invalid arguments");
     *out = nullptr;
+    ScratchScope scratch;
     cpm_opset_s *o = new cpm_opset_s();
     o->tube = t;
     int rc = build_base(o);
@@ -2146,6 +2153,7 @@ struct PlotExtras {
 };
 
 static int plot_interp_rows(cpm_opset_t op, int64_t n, const double *xp, int64_t *cols, double *vals, PlotExtras &ex) {
+    ScratchScope scratch;
     CPM_TRY(cpm_interp_query(op->tube, n, xp, cols, vals));
     for (int64_t e = 0; e < 64 * n; ++e)
         if (cols[e] < 0) return fail(CPM_ERR_BASEPOINT_OUTSIDE_TUBE, "plot interpolation stencil leaves the tube");
@@ -2160,7 +2168,7 @@ static int plot_interp_rows(cpm_opset_t op, int64_t n, const double *xp, int64_t
     bool need_normals = false, need_xn = false;
     for (int c = 0; c < n_ibc; ++c)
         if (!op->ibc_desc[c].use_cp_diff_directions) (op->ibc_desc[c].use_Jcp_surface_normals ? need_normals : need_xn) = true;
-    DBuf<double> dn, dnx;
+    TBuf<double> dn, dnx;
     const double *normals_dev = op->normals.p;
     if (need_normals) {
         if (op->normals.n >= (size_t)(3 * N)) {
@@ -2175,7 +2183,7 @@ static int plot_interp_rows(cpm_opset_t op, int64_t n, const double *xp, int64_t
         normals_x = unoriented_normals(ht);
         CPM_TRY(dnx.upload(normals_x));
     }
-    DBuf<double> xdev;
+    TBuf<double> xdev;
     CPM_TRY(xdev.alloc(3 * N));
     k_node_coords<<<(unsigned)((N + 255) / 256), 256, 0, stream()>>>(N, t->key.p, t->g.xstart, t->g.dx, xdev.p);
     CPM_CUDA_TRY(cudaGetLastError());
@@ -2185,7 +2193,7 @@ static int plot_interp_rows(cpm_opset_t op, int64_t n, const double *xp, int64_t
         CPM_TRY(build_ibc_data(t, ht, op->ibc_desc[c], op->ibc_desc[c].use_Jcp_surface_normals ? normals_dev : dnx.p, xdev,
                                ovr ? &ovr->ibc[c] : nullptr, ovr ? &ovr->surface : nullptr, ibs[c]));
     std::vector<double> hx(xp, xp + 3 * n);
-    DBuf<double> dxp;
+    TBuf<double> dxp;
     CPM_TRY(dxp.upload(hx));
     // per IBC: the points within 2r of it and their tagging directions
     std::vector<std::vector<int64_t>> sub(n_ibc, std::vector<int64_t>(n, -1));
@@ -2194,7 +2202,7 @@ static int plot_interp_rows(cpm_opset_t op, int64_t n, const double *xp, int64_t
         const cpm_surface_desc &desc = op->ibc_desc[c];
         SurfaceObj s;
         CPM_TRY(surface_init(s, &desc, r));
-        DBuf<double> dcp, dd;
+        TBuf<double> dcp, dd;
         CPM_TRY(dcp.alloc(3 * n));
         CPM_TRY(dd.alloc(n));
         CPM_TRY(closest_points_dev(s.params(), n, dxp.p, dcp.p, dd.p, 2.0 * r * (1.0 + 1e-12)));

@@ -420,7 +420,7 @@ int surface_init(SurfaceObj &s, const cpm_surface_desc *d, double cell_h) {
     s.mesh.nprims = d->nprims;
     CPM_TRY(s.mesh.verts.upload(d->verts, (size_t)d->nverts * 3));
     CPM_TRY(s.mesh.prims.upload(prims));
-    DBuf<int32_t> counts;
+    TBuf<int32_t> counts;
     CPM_TRY(counts.alloc(ncell));
     CPM_TRY(counts.zero());
     int bs = 128;
@@ -681,13 +681,13 @@ static uint32_t spread3(uint32_t v) {
 
 // Shared tail of both build entry points: candidate slots with cp/dist/band on
 // the device -> connectivity -> brick tables -> nodes -> weights.
-static int finish_build(cpm_tube_s *t, const std::vector<uint32_t> &cand_h, std::vector<int32_t> &cmap_h, DBuf<uint32_t> &cand,
-                        DBuf<double> &ccp, DBuf<double> &cdist, DBuf<uint8_t> &band, const int seed[3]) {
+static int finish_build(cpm_tube_s *t, const std::vector<uint32_t> &cand_h, std::vector<int32_t> &cmap_h, TBuf<uint32_t> &cand,
+                        TBuf<double> &ccp, TBuf<double> &cdist, TBuf<uint8_t> &band, const int seed[3]) {
     const GridParams &g = t->g;
     const int64_t nc = (int64_t)cand_h.size();
     const int bs = 256;
     for (int d = 0; d < 3; ++d) t->seed[d] = seed[d];
-    DBuf<int32_t> cmap, parent, err;
+    TBuf<int32_t> cmap, parent, err;
     CPM_TRY(cmap.upload(cmap_h));
     CPM_TRY(parent.alloc((size_t)nc * 64));
     CPM_TRY(err.alloc(1));
@@ -709,11 +709,11 @@ static int finish_build(cpm_tube_s *t, const std::vector<uint32_t> &cand_h, std:
     CPM_TRY(parent.download(par, (size_t)nc * 64));
     int root = (int)seed_slot;
     for (int it = 0; it < (1 << 26) && par[root] != root; ++it) root = par[root];
-    DBuf<uint64_t> mask;
+    TBuf<uint64_t> mask;
     CPM_TRY(mask.alloc((size_t)nc));
     k_tube_mask<<<(unsigned)((nc + bs - 1) / bs), bs, 0, stream()>>>(nc, band.p, parent.p, root, mask.p, err.p);
     CPM_CUDA_TRY(cudaGetLastError());
-    DBuf<unsigned long long> vcount;
+    TBuf<unsigned long long> vcount;
     CPM_TRY(vcount.alloc(1));
     CPM_TRY(vcount.zero());
     k_count_visited<<<gs, bs, 0, stream()>>>(cv, nc, cand.p, mask.p, vcount.p);
@@ -755,7 +755,7 @@ static int finish_build(cpm_tube_s *t, const std::vector<uint32_t> &cand_h, std:
     CPM_TRY(t->bmap.upload(bmap));
     CPM_TRY(t->bstart.upload(bstart));
     CPM_TRY(t->bmask.upload(bmask));
-    DBuf<int32_t> crank;
+    TBuf<int32_t> crank;
     CPM_TRY(crank.upload(cand_rank));
     CPM_TRY(t->key.alloc(total));
     CPM_TRY(t->cp.alloc(3 * total));
@@ -830,8 +830,8 @@ __global__ void k_seed(SurfaceParams s, GridParams g, const SeedBest *__restrict
 
 // the tube's seed node, into host memory (waits)
 static int find_seed(const SurfaceParams &sp, const GridParams &g, std::vector<int32_t> &sh) {
-    DBuf<int32_t> seed;
-    DBuf<SeedBest> best;
+    TBuf<int32_t> seed;
+    TBuf<SeedBest> best;
     CPM_TRY(seed.alloc(3));
     const bool mesh = sp.kind == CPM_TRIANGULATION || sp.kind == CPM_POLYLINE;
     if (mesh) {
@@ -850,6 +850,7 @@ using namespace cpm;
 extern "C" int cpm_tube_build(const cpm_surface_desc *surface, int32_t p, double dx, cpm_tube_t *out) {
     if (!out) return fail(CPM_ERR_INVALID_ARG, "null output handle");
     *out = nullptr;
+    ScratchScope scratch;
     cpm_tube_s *t = new cpm_tube_s();
     auto bail = [&](int rc) {
         delete t;
@@ -861,7 +862,7 @@ extern "C" int cpm_tube_build(const cpm_surface_desc *surface, int32_t p, double
     SurfaceParams sp = t->surf.params();
     const int bs = 256;
     int64_t nb3 = (int64_t)g.NB * g.NB * g.NB;
-    DBuf<int32_t> flag;
+    TBuf<int32_t> flag;
     if ((rc = flag.alloc(nb3))) return bail(rc);
     double thresh = g.radius + g.dx + 1.5 * std::sqrt(3.0) * g.dx + 1e-9 * (1.0 + g.radius);
     k_brick_candidates<<<(unsigned)((nb3 + bs - 1) / bs), bs, 0, stream()>>>(sp, g, thresh, flag.p);
@@ -877,9 +878,9 @@ extern "C" int cpm_tube_build(const cpm_surface_desc *surface, int32_t p, double
             cand_h.push_back(pack3(bi, bj, bk));
         }
     int64_t nc = (int64_t)cand_h.size();
-    DBuf<uint32_t> cand;
-    DBuf<double> ccp, cdist;
-    DBuf<uint8_t> band;
+    TBuf<uint32_t> cand;
+    TBuf<double> ccp, cdist;
+    TBuf<uint8_t> band;
     if ((rc = cand.upload(cand_h)) || (rc = ccp.alloc(3 * nc * 64)) || (rc = cdist.alloc(nc * 64)) || (rc = band.alloc(nc * 64)))
         return bail(rc);
     k_candidate_nodes<<<(unsigned)((nc * 64 + bs - 1) / bs), bs, 0, stream()>>>(sp, g, nc, cand.p, ccp.p, cdist.p, band.p);
@@ -894,6 +895,7 @@ extern "C" int cpm_tube_build_from_cp(const cpm_surface_desc *surface, int32_t p
                                       const double *cp, const double *dist, cpm_tube_t *out) {
     if (!out || n <= 0 || !keys || !cp || !dist) return fail(CPM_ERR_INVALID_ARG, "invalid arguments");
     *out = nullptr;
+    ScratchScope scratch;
     cpm_tube_s *t = new cpm_tube_s();
     auto bail = [&](int rc) {
         delete t;
@@ -932,9 +934,9 @@ extern "C" int cpm_tube_build_from_cp(const cpm_surface_desc *surface, int32_t p
     // use the device closest point of the corner, as cpm_tube_build does.
     std::vector<int32_t> sh;
     if ((rc = find_seed(t->surf.params(), g, sh))) return bail(rc);
-    DBuf<uint32_t> cand;
-    DBuf<double> ccp, cdist;
-    DBuf<uint8_t> band;
+    TBuf<uint32_t> cand;
+    TBuf<double> ccp, cdist;
+    TBuf<uint8_t> band;
     if ((rc = cand.upload(cand_h)) || (rc = ccp.upload(ccp_h)) || (rc = cdist.upload(cdist_h)) || (rc = band.upload(band_h)))
         return bail(rc);
     int sd[3] = {sh[0], sh[1], sh[2]};
@@ -1006,7 +1008,7 @@ extern "C" int cpm_tube_export(cpm_tube_t t, int64_t *rec, double *x, double *cp
         std::copy(h.begin(), h.end(), w);
     }
     if (nbr) {
-        DBuf<int64_t> d;
+        TBuf<int64_t> d;
         CPM_TRY(d.alloc(6 * N));
         k_tube_export_nbr<<<(unsigned)((N + 255) / 256), 256, 0, stream()>>>(t->view(), N, t->key.p, d.p);
         CPM_CUDA_TRY(cudaGetLastError());
@@ -1074,10 +1076,11 @@ __global__ void k_interp_rows(BrickView bv, int64_t n, const uint32_t *__restric
 extern "C" int cpm_interp_query(cpm_tube_t t, int64_t n, const double *xq, int64_t *cols, double *vals) {
     if (!t || n < 0 || (n > 0 && (!xq || !cols || !vals))) return fail(CPM_ERR_INVALID_ARG, "invalid arguments");
     if (n == 0) return 0;
-    DBuf<double> dx, dw, dv;
-    DBuf<uint32_t> db;
-    DBuf<int64_t> dc;
-    DBuf<int32_t> err;
+    ScratchScope scratch;
+    TBuf<double> dx, dw, dv;
+    TBuf<uint32_t> db;
+    TBuf<int64_t> dc;
+    TBuf<int32_t> err;
     CPM_TRY(dx.upload(xq, 3 * n));
     CPM_TRY(db.alloc(n));
     CPM_TRY(dw.alloc(12 * n));
@@ -1110,9 +1113,10 @@ extern "C" int cpm_closest_points(const cpm_surface_desc *surface, int64_t n, co
                                   double *dist) {
     if (!surface || n < 0 || (n > 0 && (!x || !cp || !dist))) return fail(CPM_ERR_INVALID_ARG, "closest_points: invalid arguments");
     if (n == 0) return 0;
+    ScratchScope scratch;
     SurfaceObj s;
     CPM_TRY(surface_init(s, surface, max_dist > 0 ? max_dist : 0.0));
-    DBuf<double> dx, dcp, dd;
+    TBuf<double> dx, dcp, dd;
     CPM_TRY(dx.upload(x, 3 * (size_t)n));
     CPM_TRY(dcp.alloc(3 * (size_t)n));
     CPM_TRY(dd.alloc((size_t)n));
