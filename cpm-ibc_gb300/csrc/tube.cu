@@ -377,9 +377,102 @@ __global__ void k_closest_points(SurfaceParams s, int64_t n, const double *__res
     dist[i] = d;
 }
 
+// A warp per point, for few points or points far from each other (the projections
+// of an IBC's DOF nodes come in the order of the tagging walk): the lanes share out
+// the primitives of each ring of cells, or of the whole mesh, first to bound the
+// distance by the spheres, then to test those that can be nearer.  The same rings,
+// arithmetic and choice as cp_mesh.  Lane by lane 6,700 projections took 2.4 ms.
+constexpr int64_t FEW_POINTS = 32768;  // a warp each; more are searched 32 to a warp
+__global__ void __launch_bounds__(128) k_closest_points_few(SurfaceParams s, int64_t n, const double *__restrict__ xs,
+                                                            double *__restrict__ cp, double *__restrict__ dist, double max_dist) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i0 >= n) return;
+    const double x[3] = {xs[3 * i0], xs[3 * i0 + 1], xs[3 * i0 + 2]};
+    const float xf[3] = {(float)x[0], (float)x[1], (float)x[2]};
+    const float slack = 2e-7f * (fabsf(xf[0]) + fabsf(xf[1]) + fabsf(xf[2]));  // x's rounding to FP32
+    float above = CUDART_INF_F;  // the distance is at most this
+    double best2 = 1e300;
+    long long bestp = -1;
+    // primitives items[t0 .. t1), or t0 .. t1 themselves
+    auto walk = [&](const int32_t *items, int64_t t0, int64_t t1, int pass) {
+        for (int64_t t = t0 + lane; t < t1; t += 32) {
+            const int64_t p = items ? __ldg(items + t) : t;
+            const float4 b = __ldg(s.sph + p);
+            const float e0 = xf[0] - b.x, e1 = xf[1] - b.y, e2 = xf[2] - b.z, d2 = e0 * e0 + e1 * e1 + e2 * e2;
+            if (pass == 0) {
+                above = fminf(above, (sqrtf(d2) + b.w) * 1.00001f + slack);
+                continue;
+            }
+            const float far = above + slack + b.w;
+            if (d2 > 1.00001f * (far * far)) continue;
+            double q[3];
+            closest_on_prim(s, p, x, q);
+            const double dd[3] = {x[0] - q[0], x[1] - q[1], x[2] - q[2]}, q2 = dot3(dd, dd);
+            if (q2 < best2 || (q2 == best2 && p < bestp)) {
+                best2 = q2;
+                bestp = p;
+                above = fminf(above, (float)sqrt(q2) * 1.00001f + slack);
+            }
+        }
+    };
+    auto share_bound = [&] {
+        for (int o = 16; o > 0; o >>= 1) above = fminf(above, __shfl_xor_sync(ALL, above, o));
+    };
+    auto share_best = [&] {
+        for (int o = 16; o > 0; o >>= 1) {
+            const double d = __shfl_xor_sync(ALL, best2, o);
+            const long long p = __shfl_xor_sync(ALL, bestp, o);
+            if (p >= 0 && (d < best2 || (d == best2 && (bestp < 0 || p < bestp)))) {
+                best2 = d;
+                bestp = p;
+            }
+        }
+    };
+    if (!isfinite(max_dist)) {
+        walk(nullptr, 0, s.nprims, 0);
+        share_bound();
+        walk(nullptr, 0, s.nprims, 1);
+        share_best();
+    } else {
+        int c[3];
+        for (int d = 0; d < 3; ++d) c[d] = (int)fmin(fmax(floor((x[d] - s.glo[d]) / s.gh), 0.0), (double)(s.gn[d] - 1));
+        const int maxring = max(s.gn[0], max(s.gn[1], s.gn[2]));
+        for (int ring = 0; ring <= maxring; ++ring) {
+            const int k0 = max(c[2] - ring, 0), k1 = min(c[2] + ring, s.gn[2] - 1);
+            for (int pass = 0; pass < 2; ++pass) {
+                for (int i = max(c[0] - ring, 0); i <= min(c[0] + ring, s.gn[0] - 1); ++i)
+                    for (int j = max(c[1] - ring, 0); j <= min(c[1] + ring, s.gn[1] - 1); ++j) {
+                        const int32_t *start = s.cell_start + ((size_t)i * s.gn[1] + j) * s.gn[2];
+                        if (max(abs(i - c[0]), abs(j - c[1])) == ring) {  // a whole run of cells along k
+                            walk(s.cell_items, __ldg(start + k0), __ldg(start + k1 + 1), pass);
+                        } else {  // the ring's two cells along k
+                            if (c[2] - ring >= 0) walk(s.cell_items, __ldg(start + k0), __ldg(start + k0 + 1), pass);
+                            if (c[2] + ring < s.gn[2]) walk(s.cell_items, __ldg(start + k1), __ldg(start + k1 + 1), pass);
+                        }
+                    }
+                if (pass == 0) share_bound();
+            }
+            share_best();
+            const double reach = ring * s.gh;
+            if (best2 <= reach * reach || reach > max_dist) break;
+        }
+    }
+    double q[3] = {0, 0, 0};
+    if (bestp >= 0) closest_on_prim(s, bestp, x, q);
+    if (lane < 3) cp[3 * i0 + lane] = lane == 0 ? q[0] : lane == 1 ? q[1] : q[2];
+    if (lane == 0) dist[i0] = sqrt(best2);
+}
+
 int closest_points_dev(const SurfaceParams &sp, int64_t n, const double *x, double *cp, double *dist, double max_dist) {
     if (n <= 0) return 0;
     int bs = 128;
+    if ((sp.kind == CPM_TRIANGULATION || sp.kind == CPM_POLYLINE) && n <= FEW_POINTS) {
+        k_closest_points_few<<<(unsigned)((32 * n + bs - 1) / bs), bs, 0, stream()>>>(sp, n, x, cp, dist, max_dist);
+        CPM_CUDA_TRY(cudaGetLastError());
+        return 0;
+    }
     k_closest_points<<<(unsigned)((n + bs - 1) / bs), bs, 0, stream()>>>(sp, n, x, cp, dist, max_dist);
     CPM_CUDA_TRY(cudaGetLastError());
     return 0;

@@ -46,7 +46,14 @@ def test_culled_search_finds_the_nearest(shape, shift):
     want = _distance(v, f, x)
     bb = workloads.mesh_bbox(v + shift)
     for max_dist in (0.0, 0.1):
-        cp, dist = cg.closest_points(cg.desc(kind, (), bb, verts=v + shift, prims=f), x + shift, max_dist)
+        d = cg.desc(kind, (), bb, verts=v + shift, prims=f)
+        cp, dist = cg.closest_points(d, x + shift, max_dist)
+        # more points than are searched by a warp each: near each other 32 at a time, then scattered
+        for many in (np.repeat(np.arange(len(x)), 160), np.tile(np.arange(len(x)), 160)):
+            cpm, distm = cg.closest_points(d, (x + shift)[many], max_dist)
+            ok = dist[many] <= (max_dist or np.inf)
+            assert np.array_equal(distm[ok], dist[many][ok]) and np.array_equal(cpm[ok], cp[many][ok])
+            assert np.all(distm[~ok] > max_dist)
         near = np.ones(len(x), bool) if max_dist == 0.0 else want <= max_dist
         tol = 1e-13 + 4 * shift * 2.0 ** -52 * 4
         assert np.all(np.abs(dist - want)[near] <= tol), np.max(np.abs(dist - want)[near])
