@@ -100,6 +100,15 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// 4 bytes, or zeros
+__device__ __forceinline__ void cp_async4(void *dst, const void *src, bool there) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 template <class... P, class... A>
 static void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
@@ -423,83 +432,133 @@ __device__ __forceinline__ void e_ident32(const OpView<T> &op, int warp, int lan
 // by plane (16 columns each) and keeps each pair of rows' sum in registers
 // (f32x2): plane i adds wx_i (sum_j wy_j sum_k wz_k x_ijk) in plane order, with
 // no block-level synchronisation and no shared partial sums.  Rows EW_ROWS at a
-// time; weights staged pair-interleaved in the warp's shared memory.  Identity
-// rows copied warp per row.  ph < 0: every slot.
-constexpr int EW_ROWS = 8;
-__global__ void __launch_bounds__(128) k_epass32w(OpView<float> op, const Slot *sl, int ph, int nb_plain,
+// time.  Identity rows copied warp per row.  ph < 0: every slot.
+// Bound by the latency of the gathers and the warps in flight (issue slots half
+// used, LSU 60 %, L2 reads at 6.6 TB/s on the torus at dx 0.01).  So the group's
+// tables (columns, pair-interleaved weights) are copied one group ahead into the
+// warp's shared memory, which takes no registers: reading them when they were due
+// put two more latencies into each plane, and holding them in registers spills at
+// eight blocks per SM.  FP32 apply 84 -> 75 us on the two-circle sphere at dx
+// 0.025, 479 -> 407 us on the torus; at 6 / 7 / 9 blocks 81 / 77.5 / 78 us.
+constexpr int EW_ROWS = 8, EW_BPS = 8;
+// what a warp of the pass reads of a group's tables: 64 columns, and the weights of
+// at most EW_ROWS rows in pairs, zeros for the odd row of a last pair
+struct EwStage {
+    alignas(16) int col[64];
+    alignas(16) float w[EW_ROWS * 12];
+    __device__ __forceinline__ void fetch(const OpView<float> &op, int64_t g, int c0, int nr, int lane) {
+        if (lane < 16) cp_async16(col + 4 * lane, op.gcols + 64 * g + 4 * lane);
+#pragma unroll
+        for (int m = 0; m < EW_ROWS * 12 / 32; ++m) {
+            const int e = lane + 32 * m, q = e / 12, c = e - 12 * q;
+            cp_async4(w + 24 * (q >> 1) + 2 * c + (q & 1), op.w_ord + 12 * (size_t)c0 + (q < nr ? e : 0), q < nr);
+        }
+        cp_async_commit();
+    }
+};
+__global__ void __launch_bounds__(128, EW_BPS) k_epass32w(OpView<float> op, const Slot *sl, int ph, int nb_plain,
                                                   const float *x, float *t) {
-    pdl_wait();
-    __shared__ __align__(16) float sw[4][EW_ROWS * 12];
+    __shared__ EwStage stage[4][2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    EwStage *st = stage[warp];
+    const GroupLoop gl(op, nb_plain, 4, warp);
+    int64_t g = gl.g;
+    int c0 = 0, p1 = 0, n0 = 0, n1 = 0;  // the rows of g, and of g + step
+    if (g < gl.end) {
+        c0 = __ldg(op.grp + g);
+        p1 = __ldg(op.grp + g + 1);
+        st[0].fetch(op, g, c0, p1 - c0, lane);
+        if (g + gl.step < gl.end) {
+            n0 = __ldg(op.grp + g + gl.step);
+            n1 = __ldg(op.grp + g + gl.step + 1);
+        }
+    }
+    pdl_wait();
     const bool act = (ph < 0) || sl[lane].phase == ph;
-    if (!__any_sync(FULL, act)) return;  // the same 32 slots in every warp: block-uniform
-    float *w = sw[warp];
+    if (!__any_sync(FULL, act)) {  // the same 32 slots in every warp: block-uniform
+        cp_async_wait();
+        return;
+    }
     const float *__restrict__ xl = x + lane;
-    for (GroupLoop gl(op, nb_plain, 4, warp); gl.g < gl.end; gl.g += gl.step) {
-        const int64_t g = gl.g;
-        const int p0 = op.grp[g], p1 = op.grp[g + 1];
-        for (int c0 = p0; c0 < p1; c0 += EW_ROWS) {
-            // rows in pairs, the odd row of a last pair with zero weights
-            const int nr = min(p1 - c0, EW_ROWS), np = (nr + 1) >> 1;
-            __syncwarp();
-            for (int e = lane; e < 24 * np; e += 32) {
-                const int q = e / 12, c = e - 12 * q;
-                w[24 * (q >> 1) + 2 * c + (q & 1)] = q < nr ? op.w_ord[12 * (size_t)(c0 + q) + c] : 0.f;
+    int b = 0;
+    while (g < gl.end) {
+        const int nr = min(p1 - c0, EW_ROWS), np = (nr + 1) >> 1;
+        const int at = c0;
+        cp_async_wait();
+        __syncwarp();
+        if (c0 + EW_ROWS < p1) {
+            c0 += EW_ROWS;
+        } else {
+            g += gl.step;
+            c0 = n0;
+            p1 = n1;
+            if (g + gl.step < gl.end) {
+                n0 = __ldg(op.grp + g + gl.step);
+                n1 = __ldg(op.grp + g + gl.step + 1);
             }
-            const int row = lane < nr ? op.ord[c0 + lane] : 0;  // lane q: row q of the chunk
-            const int fl = lane < nr ? op.fl_ord[c0 + lane] & F_TERMS : 0;
-            const bool terms = __any_sync(FULL, fl != 0);
-            uint64_t acc[EW_ROWS / 2];
+        }
+        if (g < gl.end) st[b ^ 1].fetch(op, g, c0, p1 - c0, lane);
+        const int row = lane < nr ? __ldg(op.ord + at + lane) : 0;  // lane q: row q of the chunk
+        const int fl = lane < nr ? __ldg(op.fl_ord + at + lane) & F_TERMS : 0;
+        uint64_t acc[EW_ROWS / 2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                int col[16];
-                float xb[16];
-                e_group_cols(op.gcols, g, i, col);
-                // every lane loads (inactive slots' values are computed and not stored);
-                // the rows are whole 128-byte lines either way
+        for (int i = 0; i < 4; ++i) {
+            int col[16];
+            float xb[16];
 #pragma unroll
-                for (int q = 0; q < 16; ++q) xb[q] = xl[(uint32_t)col[q] * 32u];
-                uint64_t x2[16];
-#pragma unroll
-                for (int q = 0; q < 16; ++q) x2[q] = f2_pack(xb[q], xb[q]);
-#pragma unroll
-                for (int p = 0; p < EW_ROWS / 2; ++p)
-                    if (p < np) {
-                        const float *wp = w + 24 * p;
-                        const uint64_t wx2 = *(const uint64_t *)(wp + 2 * i);
-                        const ulonglong2 y01 = *(const ulonglong2 *)(wp + 8), y23 = *(const ulonglong2 *)(wp + 12);
-                        const ulonglong2 z01 = *(const ulonglong2 *)(wp + 16), z23 = *(const ulonglong2 *)(wp + 20);
-                        const uint64_t wy2[4] = {y01.x, y01.y, y23.x, y23.y}, wz2[4] = {z01.x, z01.y, z23.x, z23.y};
-                        uint64_t ay2 = 0ull;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint64_t az2 = f2_mul(wz2[0], x2[4 * j]);
-                            az2 = f2_fma(wz2[1], x2[4 * j + 1], az2);
-                            az2 = f2_fma(wz2[2], x2[4 * j + 2], az2);
-                            az2 = f2_fma(wz2[3], x2[4 * j + 3], az2);
-                            ay2 = j == 0 ? f2_mul(wy2[0], az2) : f2_fma(wy2[j], az2, ay2);
-                        }
-                        const uint64_t part = f2_mul(wx2, ay2);
-                        acc[p] = i == 0 ? part : f2_add(acc[p], part);
-                    }
+            for (int v = 0; v < 4; ++v) {
+                const int4 c = ((const int4 *)st[b].col)[4 * i + v];
+                col[4 * v] = c.x;
+                col[4 * v + 1] = c.y;
+                col[4 * v + 2] = c.z;
+                col[4 * v + 3] = c.w;
             }
+            // every lane loads (inactive slots' values are computed and not stored);
+            // the rows are whole 128-byte lines either way
+#pragma unroll
+            for (int q = 0; q < 16; ++q) xb[q] = xl[(uint32_t)col[q] * 32u];
+            uint64_t x2[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) x2[q] = f2_pack(xb[q], xb[q]);
 #pragma unroll
             for (int p = 0; p < EW_ROWS / 2; ++p)
-                if (2 * p < nr) {
-                    float lo, hi;
-                    f2_unpack(acc[p], lo, hi);
-                    const int r0 = __shfl_sync(FULL, row, 2 * p), r1 = __shfl_sync(FULL, row, 2 * p + 1);
-                    if (terms) {
-                        const int f0 = __shfl_sync(FULL, fl, 2 * p), f1 = __shfl_sync(FULL, fl, 2 * p + 1);
-                        if (f0) lo = e_row_terms<float, 32>(op, (uint8_t)f0, r0, lane, lo, x);
-                        if (f1) hi = e_row_terms<float, 32>(op, (uint8_t)f1, r1, lane, hi, x);
+                if (p < np) {
+                    const float *wp = st[b].w + 24 * p;
+                    const uint64_t wx2 = *(const uint64_t *)(wp + 2 * i);
+                    const ulonglong2 y01 = *(const ulonglong2 *)(wp + 8), y23 = *(const ulonglong2 *)(wp + 12);
+                    const ulonglong2 z01 = *(const ulonglong2 *)(wp + 16), z23 = *(const ulonglong2 *)(wp + 20);
+                    const uint64_t wy2[4] = {y01.x, y01.y, y23.x, y23.y}, wz2[4] = {z01.x, z01.y, z23.x, z23.y};
+                    uint64_t ay2 = 0ull;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        uint64_t az2 = f2_mul(wz2[0], x2[4 * j]);
+                        az2 = f2_fma(wz2[1], x2[4 * j + 1], az2);
+                        az2 = f2_fma(wz2[2], x2[4 * j + 2], az2);
+                        az2 = f2_fma(wz2[3], x2[4 * j + 3], az2);
+                        ay2 = j == 0 ? f2_mul(wy2[0], az2) : f2_fma(wy2[j], az2, ay2);
                     }
-                    if (act) {
-                        t[(uint32_t)r0 * 32u + lane] = lo;
-                        if (2 * p + 1 < nr) t[(uint32_t)r1 * 32u + lane] = hi;
-                    }
+                    const uint64_t part = f2_mul(wx2, ay2);
+                    acc[p] = i == 0 ? part : f2_add(acc[p], part);
                 }
         }
+        const bool terms = __any_sync(FULL, fl != 0);
+#pragma unroll
+        for (int p = 0; p < EW_ROWS / 2; ++p)
+            if (2 * p < nr) {
+                float lo, hi;
+                f2_unpack(acc[p], lo, hi);
+                const int r0 = __shfl_sync(FULL, row, 2 * p), r1 = __shfl_sync(FULL, row, 2 * p + 1);
+                if (terms) {
+                    const int f0 = __shfl_sync(FULL, fl, 2 * p), f1 = __shfl_sync(FULL, fl, 2 * p + 1);
+                    if (f0) lo = e_row_terms<float, 32>(op, (uint8_t)f0, r0, lane, lo, x);
+                    if (f1) hi = e_row_terms<float, 32>(op, (uint8_t)f1, r1, lane, hi, x);
+                }
+                if (act) {
+                    t[(uint32_t)r0 * 32u + lane] = lo;
+                    if (2 * p + 1 < nr) t[(uint32_t)r1 * 32u + lane] = hi;
+                }
+            }
+        b ^= 1;
     }
     e_ident32(op, warp, lane, act, x, t);
 }
@@ -809,12 +868,27 @@ static void slot_epatch(const OpView<T> &op, const Slot *sl, int ph, const T *x,
     launch_after(k_slot_epatch32<T>, (unsigned)blocks, 128, st, op, sl, ph, x, t);
 }
 
-// default launch shapes of the 32-slot E passes (blocks per SM caps of the
-// grid-stride loops over the groups without and with moved columns).  On the
-// sphere with two circles at dx 0.025 16 blocks took 81.4 us for the FP32 apply and
-// 386 us for the FP64 one (32: 82.8, 391; 64: 83.8, 399; 8 in FP64: 390); the
-// passes over groups with moved columns do not mind.
-constexpr int E32_BPS = 16, PATCH_BPS = 64, E64_BPS = 16;
+// Default launch shapes of the 32-slot E passes, as caps in blocks per SM of the
+// grid-stride loops.  Groups differ in rows, so the warps' ends are level only if
+// each has few of them; with a handful the tables read ahead no longer pay.  So
+// the cap doubles from 8, what an SM holds at once, until a warp has at most
+// E_GROUPS groups.  FP32 apply at 8 / 16 / 32 / 64: two-circle sphere at dx 0.025
+// (15 groups a warp at 8) 75.3 / 75.5 / 78.6 / 80.1 us, torus at 0.01
+// 469 / 432 / 417 / 407 us; FP64 on the sphere (15 a pair of warps at 16) 390 / 386 / 391 / 399 us.
+// The passes over groups with moved columns do not mind.
+constexpr int E_GROUPS = 16, E_BPS_MIN = 8, E_BPS_MAX = 64, PATCH_BPS = 64;
+
+// groups a block takes at once: four warps with one (FP32) or two pairs (FP64)
+template <class T>
+constexpr int groups_per_block() {
+    return sizeof(T) == 4 ? 4 : 2;
+}
+template <class T>
+static inline int default_bps(int64_t n) {
+    int bps = E_BPS_MIN;
+    while (bps < E_BPS_MAX && n > (int64_t)E_GROUPS * groups_per_block<T>() * bps * sm_count()) bps *= 2;
+    return bps;
+}
 
 // kernels one E pass of x launches
 template <class T, int K>
@@ -822,10 +896,10 @@ static inline int epass_kernels(const OpView<T> &op, const T *) {
     return (K == 32 && op.n_sp_rows > 0) ? 2 : 1;
 }
 
-// blocks of a 32-slot pass over n groups: four a block (FP32) or two (FP64)
+// blocks of a 32-slot pass over n groups
 template <class T>
 static inline int group_blocks(int64_t n, int bps) {
-    constexpr int per = sizeof(T) == 4 ? 4 : 2;
+    constexpr int per = groups_per_block<T>();
     return (int)std::min<int64_t>((n + per - 1) / per, (int64_t)bps * sm_count());
 }
 
@@ -833,8 +907,8 @@ template <class T, int K>
 static void launch_epass(const OpView<T> &op, const Slot *sl, int ph, const T *x, T *t, cudaStream_t st) {
     static_assert(K == 1 || K == 32, "slot widths 1 and 32");
     if constexpr (K == 32) {
-        const int bps = sizeof(T) == 4 ? (op.e32_bps > 0 ? op.e32_bps : E32_BPS) : (op.e64_bps > 0 ? op.e64_bps : E64_BPS);
-        const int plain = group_blocks<T>(op.n_grp_plain, bps);
+        const int set = sizeof(T) == 4 ? op.e32_bps : op.e64_bps;
+        const int plain = group_blocks<T>(op.n_grp_plain, set > 0 ? set : default_bps<T>(op.n_grp_plain));
         const int crossing = group_blocks<T>(op.n_grp - op.n_grp_plain, op.patch_bps > 0 ? op.patch_bps : PATCH_BPS);
         const unsigned blocks = (unsigned)std::max(1, plain + crossing);
         if constexpr (sizeof(T) == 4)
@@ -2970,7 +3044,7 @@ extern "C" int cpm_opset_autotune(cpm_opset_t op, int32_t reps, int32_t with_fp6
     };
     // one range of groups alone: the others get no block
     if (v32.n_grp_plain > 0) {
-        pick(e32c, 8, E32_BPS, [&](int bps) {
+        pick(e32c, 8, default_bps<float>(v32.n_grp_plain), [&](int bps) {
             const int blocks = group_blocks<float>(v32.n_grp_plain, bps);
             k_epass32w<<<blocks, 128, 0, st>>>(v32, nullptr, -1, blocks, x32.p, t32.p);
         }, res.e32_us, res.e32_default_us, res.e32_blocks_per_sm);
@@ -2982,7 +3056,7 @@ extern "C" int cpm_opset_autotune(cpm_opset_t op, int32_t reps, int32_t with_fp6
     }
     if (with_fp64 && op->n_grp_plain > 0) {
         const OpView<double> v64 = op->view<double>();
-        pick(e64c, 5, E64_BPS, [&](int bps) {
+        pick(e64c, 5, default_bps<double>(v64.n_grp_plain), [&](int bps) {
             const int blocks = group_blocks<double>(v64.n_grp_plain, bps);
             k_epass32x<<<blocks, 128, 0, st>>>(v64, nullptr, -1, blocks, x64.p, t64.p);
         }, res.e64_us, res.e64_default_us, res.e64_blocks_per_sm);
