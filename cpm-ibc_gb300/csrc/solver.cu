@@ -439,8 +439,11 @@ __device__ __forceinline__ void e_ident32(const OpView<T> &op, int warp, int lan
 // warp's shared memory, which takes no registers: reading them when they were due
 // put two more latencies into each plane, and holding them in registers spills at
 // eight blocks per SM.  FP32 apply 84 -> 75 us on the two-circle sphere at dx
-// 0.025, 479 -> 407 us on the torus; at 6 / 7 / 9 blocks 81 / 77.5 / 78 us.
-constexpr int EW_ROWS = 8, EW_BPS = 8;
+// 0.025, 479 -> 407 us on the torus; at 6 / 7 / 9 blocks 81 / 77.5 / 78 us.  A
+// group's values are gathered again for each EW_ROWS of its rows: with 6 / 8 / 10 /
+// 12 the torus took 433 / 407 / 399 / 411 us (seven rows a group are usual, and
+// more sums than 10 spill).
+constexpr int EW_ROWS = 10, EW_BPS = 8;
 // what a warp of the pass reads of a group's tables: 64 columns, and the weights of
 // at most EW_ROWS rows in pairs, zeros for the odd row of a last pair
 struct EwStage {
@@ -449,9 +452,9 @@ struct EwStage {
     __device__ __forceinline__ void fetch(const OpView<float> &op, int64_t g, int c0, int nr, int lane) {
         if (lane < 16) cp_async16(col + 4 * lane, op.gcols + 64 * g + 4 * lane);
 #pragma unroll
-        for (int m = 0; m < EW_ROWS * 12 / 32; ++m) {
+        for (int m = 0; m < (EW_ROWS * 12 + 31) / 32; ++m) {
             const int e = lane + 32 * m, q = e / 12, c = e - 12 * q;
-            cp_async4(w + 24 * (q >> 1) + 2 * c + (q & 1), op.w_ord + 12 * (size_t)c0 + (q < nr ? e : 0), q < nr);
+            if (q < EW_ROWS) cp_async4(w + 24 * (q >> 1) + 2 * c + (q & 1), op.w_ord + 12 * (size_t)c0 + (q < nr ? e : 0), q < nr);
         }
         cp_async_commit();
     }
@@ -873,10 +876,11 @@ static void slot_epatch(const OpView<T> &op, const Slot *sl, int ph, const T *x,
 // each has few of them; with a handful the tables read ahead no longer pay.  So
 // the cap doubles from 8, what an SM holds at once, until a warp has at most
 // E_GROUPS groups.  FP32 apply at 8 / 16 / 32 / 64: two-circle sphere at dx 0.025
-// (15 groups a warp at 8) 75.3 / 75.5 / 78.6 / 80.1 us, torus at 0.01
-// 469 / 432 / 417 / 407 us; FP64 on the sphere (15 a pair of warps at 16) 390 / 386 / 391 / 399 us.
-// The passes over groups with moved columns do not mind.
-constexpr int E_GROUPS = 16, E_BPS_MIN = 8, E_BPS_MAX = 64, PATCH_BPS = 64;
+// (27 thousand groups, 6 a warp at 8) 75.3 / 75.5 / 78.6 / 80.1 us, torus at 0.01
+// (222 thousand, 6 a warp at 64) 469 / 432 / 417 / 407 us; FP64 on the sphere (6 a
+// pair of warps at 16) 390 / 386 / 391 / 399 us.  The passes over groups with moved
+// columns do not mind.
+constexpr int E_GROUPS = 8, E_BPS_MIN = 8, E_BPS_MAX = 64, PATCH_BPS = 64;
 
 // groups a block takes at once: four warps with one (FP32) or two pairs (FP64)
 template <class T>
