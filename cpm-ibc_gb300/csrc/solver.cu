@@ -825,7 +825,13 @@ __global__ void __launch_bounds__(E1_T, 7) k_epass1(OpView<T> op, const Slot *sl
     const int64_t c = (int64_t)blockIdx.x * (E1_T / 32) + warp;
     const bool rows = blockIdx.x < row_blocks && c < op.n_chunk;
     E1Run q;
-    if (rows) e1_tables(op, c, lane, q);  // while the previous kernel ends
+    if (rows) {  // while the previous kernel ends
+        e1_tables(op, c, lane, q);
+        // the run's weights (a line a lane) on their way from DRAM while the values are
+        // gathered: 101.3 -> 92.4 us an apply on the torus at dx 0.01
+        if (sizeof(T) == 8 && lane < ((q.ch.w & 255) * 96 + 127) / 128)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)(op.w_fix + 12 * (int64_t)q.ch.y) + 128 * lane));
+    }
     pdl_wait();
     if (ph >= 0 && sl[0].phase != ph) return;
     if (rows) {
