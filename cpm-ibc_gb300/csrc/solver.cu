@@ -3052,23 +3052,30 @@ extern "C" int cpm_opset_autotune(cpm_opset_t op, int32_t reps, int32_t with_fp6
             best_us = dflt_us;
         }
     };
-    // one range of groups alone: the others get no block
+    // whole passes: the groups with moved columns fill the ends of the others, and the cap
+    // that is best without them (32 on the two-circle sphere at dx 0.025) is 2 % slower with them
+    auto pass32 = [&](int plain_bps, int crossing_bps) {
+        const int plain = group_blocks<float>(v32.n_grp_plain, plain_bps);
+        const int crossing = group_blocks<float>(v32.n_grp - v32.n_grp_plain, crossing_bps);
+        k_epass32w<<<plain + crossing, 128, 0, st>>>(v32, nullptr, -1, plain, x32.p, t32.p);
+    };
+    int plain32 = default_bps<float>(v32.n_grp_plain), crossing_bps = PATCH_BPS;
     if (v32.n_grp_plain > 0) {
-        pick(e32c, 8, default_bps<float>(v32.n_grp_plain), [&](int bps) {
-            const int blocks = group_blocks<float>(v32.n_grp_plain, bps);
-            k_epass32w<<<blocks, 128, 0, st>>>(v32, nullptr, -1, blocks, x32.p, t32.p);
-        }, res.e32_us, res.e32_default_us, res.e32_blocks_per_sm);
+        pick(e32c, 8, plain32, [&](int bps) { pass32(bps, PATCH_BPS); }, res.e32_us, res.e32_default_us,
+             res.e32_blocks_per_sm);
+        plain32 = res.e32_blocks_per_sm;
     }
     if (v32.n_grp > v32.n_grp_plain) {
-        pick(pc, 6, PATCH_BPS, [&](int bps) {
-            k_epass32w<<<group_blocks<float>(v32.n_grp - v32.n_grp_plain, bps), 128, 0, st>>>(v32, nullptr, -1, 0, x32.p, t32.p);
-        }, res.patch_us, res.patch_default_us, res.patch_blocks_per_sm);
+        pick(pc, 6, PATCH_BPS, [&](int bps) { pass32(plain32, bps); }, res.patch_us, res.patch_default_us,
+             res.patch_blocks_per_sm);
+        crossing_bps = res.patch_blocks_per_sm;
     }
     if (with_fp64 && op->n_grp_plain > 0) {
         const OpView<double> v64 = op->view<double>();
+        const int crossing = group_blocks<double>(v64.n_grp - v64.n_grp_plain, crossing_bps);
         pick(e64c, 5, default_bps<double>(v64.n_grp_plain), [&](int bps) {
-            const int blocks = group_blocks<double>(v64.n_grp_plain, bps);
-            k_epass32x<<<blocks, 128, 0, st>>>(v64, nullptr, -1, blocks, x64.p, t64.p);
+            const int plain = group_blocks<double>(v64.n_grp_plain, bps);
+            k_epass32x<<<plain + crossing, 128, 0, st>>>(v64, nullptr, -1, plain, x64.p, t64.p);
         }, res.e64_us, res.e64_default_us, res.e64_blocks_per_sm);
     }
     CPM_CUDA_TRY(cudaGetLastError());

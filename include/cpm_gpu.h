@@ -269,12 +269,12 @@ int cpm_apply_device(cpm_opset_t op, double m, double n, int32_t kslots, int32_t
  * counterpart in the reference, whose E is a CPU sparse product. */
 typedef struct {
     int32_t e32_blocks_per_sm, patch_blocks_per_sm, e64_blocks_per_sm;
-    float e32_us, patch_us, e64_us;                      /* the chosen shapes' mean launch times */
+    float e32_us, patch_us, e64_us;                      /* mean launch times of the whole pass */
     float e32_default_us, patch_default_us, e64_default_us; /* the defaults' */
 } cpm_tune_result;
 /* Set the shapes by hand (0: default). */
 int cpm_opset_set_launch(cpm_opset_t op, int32_t e32_blocks_per_sm, int32_t patch_blocks_per_sm, int32_t e64_blocks_per_sm);
-/* The autotuner: time each pass over candidate shapes (reps launches each, on
+/* The autotuner: time whole E passes over candidate shapes (reps launches each, on
  * scratch vectors it allocates and frees; the FP64 pass only when with_fp64)
  * on the calling thread's stream, keep the fastest with the operator (the
  * default unless another is at least 2 % faster) and report the times in
