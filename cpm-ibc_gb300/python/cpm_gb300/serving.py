@@ -43,8 +43,9 @@ from . import DIAGONAL, Geodesic, GeodesicBatch, OpSet, Server, Solver, device_i
 
 MAX_SLOTS = 32
 PROBE = 2  # requests in a surface's first mixed-precision batch
-K32_MIXED = 2.3  # 32-slot FP32 iteration (reliable updates amortised) / one-RHS FP64 iteration
-K32_FP64 = 14.0  # 32-slot FP64 iteration / one-RHS FP64 iteration
+K32_MIXED = 4.4  # 32-slot FP32 iteration (reliable updates amortised) / one-RHS FP64 iteration: 285 us / 65 us on
+# the two-circle sphere at dx 0.025
+K32_FP64 = 15.0  # 32-slot FP64 iteration / one-RHS FP64 iteration: 988 us / 65 us
 # geodesics waiting on one surface from which a batch beats solving them one by one: the
 # 32-source batch costs the same with 2 or 32 sources (FP64, lane = source), 146.9 s on the
 # torus against 6.27 s for one source alone
