@@ -642,7 +642,7 @@ def main():
     assert all(got[k][1]["status"] == 0 for k in he)
     e2e_value = replicas_value(world, n_e2e, e2e_s)
 
-    # ---- roofline of the L.E apply (FP32, 32 RHS): E pass, IBC patch rows and L pass on the library stream
+    # ---- roofline of the L.E apply (FP32, 32 RHS): E pass and L pass on the library stream
     xf = torch.randn((D, KSLOTS), dtype=torch.float32, device=dev)
     tf = torch.empty_like(xf)
     yf = torch.empty_like(xf)
@@ -754,7 +754,7 @@ def main():
                     "d2h_bytes_per_step": int(D * per_step * 8),
                     "path": f"cpm_server_submit / cpm_server_step / cpm_server_poll with host arrays, {n_e2e} requests"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": traffic, "kernel": "L.E apply (E pass + IBC patch rows + L pass), FP32, 32 RHS",
+                         "traffic": traffic, "kernel": "L.E apply (E pass + L pass), FP32, 32 RHS",
                          "apply_us": apply_s * 1e6, "alg_bytes_per_apply": alg_bytes, "peak_source": peak_src,
                          "fp32": {"achieved": fp32_achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                                   "frac": fp32_achieved / fp32_peak, "flops_per_apply": int(fp32_flops),

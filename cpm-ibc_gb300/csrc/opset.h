@@ -21,8 +21,8 @@ enum RowFlags : uint8_t {
 };
 
 // Device view of an operator set in one arithmetic type: the rows of E and L
-// (bulk stencils, IBC patches), the apply schedule (rows sorted into base
-// groups, identity rows, neighbour table) and the per-slot patches of a batch.
+// (bulk stencils, IBC patches), the apply schedule (rows sorted into groups of
+// equal columns, identity rows, neighbour table) and the per-slot patches of a batch.
 template <class T>
 struct OpView {
     BrickView bv;
