@@ -47,9 +47,9 @@ K32_MIXED = 4.4  # 32-slot FP32 iteration (reliable updates amortised) / one-RHS
 # the two-circle sphere at dx 0.025
 K32_FP64 = 15.0  # 32-slot FP64 iteration / one-RHS FP64 iteration: 988 us / 65 us
 # geodesics waiting on one surface from which a batch beats solving them one by one: the
-# 32-source batch costs the same with 2 or 32 sources (FP64, lane = source), 146.9 s on the
-# torus against 6.27 s for one source alone
-GEO_BATCH_MIN = 24
+# 32-source batch costs the same with 2 or 32 sources (FP64, lane = source), 50.1 s on the
+# torus at dx 0.01 against 1.58 s for one source alone
+GEO_BATCH_MIN = 32
 
 
 class ServedSurface:
