@@ -5,16 +5,36 @@
 // 32 x 32 + 64 -> 64 multiply-adds.  So the E sums of FP64 vectors are block
 // floating point: the 64 values of a stencil are aligned to the stencil's
 // largest exponent e as integers of 61 bits and a sign, the 1-D weights are
-// integers w 2^62, and a product keeps its 64 high bits from three multiply-adds
+// integers w 2^62, and a product keeps its high bits from three multiply-adds
 // of 32-bit halves (the product of the low halves is below the last bit).
-// Each of the three 1-D sums scales by 2^62 / 2^64, so a row ends as an integer
-// of 2^(e - 54): 2^-55 of the largest value, rounded to nearest there and once
-// more to 53 bits.  Plain FP64 rounds 84 times at 2^-53 of the running sums;
-// measured against 64-bit-exact rows the error here is the smaller one
-// (k_epass1, k_epass32x).
+// All three 1-D sums are kept in units of 2^(e - 60), two bits more than the high
+// word of the product, and stay within 62 bits: a cubic row's weights sum to at
+// most 1.25 in magnitude an axis.
+//
+// So a row is off by at most 25 units of 2^(e - 60), usually by half of one, and
+// once more by its conversion to 53 bits, where the FP64 sum rounds up to 12 times
+// at 2^-53 of the row's own terms.  It is the fixed-point sum only where that is
+// the better one: a row whose terms sum |w x| is not seen to reach 2^(e - 7) (from
+// its value, fx_small, else from its eight central terms, fx_weak) takes the FP64
+// sum.  These are rows that hardly weigh their largest value: a closest point next
+// to a grid node of small value, the steep front of a decaying field.  Host
+// restatements of 40 thousand rows a field, in units of 2^-53 sum |w x|, rms /
+// largest error:
+//   field                       FP64 sum     fixed point   rows redone
+//   noise                       0.57 / 3.5   0.21 / 1.0    none
+//   linear through zero         0.59 / 3.0   0.23 / 0.8    none
+//   the same, 7 of 10 points by
+//   a grid plane an axis        0.96 / 5.6   0.37 / 2.8    4e-3
+//   exp(-d/dx)                  0.59 / 3.8   0.24 / 1.0    none
+//   exp(-d/(0.3 dx))            0.32 / 2.4   0.30 / 2.4    0.84
+//   a factor 1e-4 a cell        0.62 / 3.8   0.61 / 3.8    0.98
+// Without that choice the last two rows are off by up to 470 and 4e6 such units.
+// In solves 0.5 to 2 % of the rows take it, at the front of the first iterates; the
+// choice costs 4 % of a solve and the rows redone 4 to 12 % (FP64, one vector at dx
+// 0.025 on the sphere 16.0 -> 17.6 ms, 32 on the torus at 0.04 82.7 -> 96.9 ms).
 //
 // A stencil with an infinity, a NaN or only values below 2^-895 (nothing is
-// left of the exponent range to align to) takes the FP64 sum instead.
+// left of the exponent range to align to) takes the FP64 sum as well.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -68,29 +88,43 @@ __device__ __forceinline__ int64_t fx_mad(int a, int b, int64_t c) {
     asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
     return d;
 }
-// (sum_k x_k w_k) / 2^64, rounded
+// (sum_k x_k w_k) / 2^62, rounded
 __device__ __forceinline__ int64_t fx_dot4(const Fx (&x)[4], const Fx (&w)[4]) {
-    int64_t c = 0x80000000ll;
+    int64_t c = 0x80000000ll >> 2, a = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) c = fx_mad(x[k].l, w[k].h, fx_mad(x[k].h, w[k].l, c));
-    int64_t a = c >> 32;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) a = fx_mad(x[k].h, w[k].h, a);
-    return a;
+    for (int k = 0; k < 4; ++k) {
+        c = fx_mad(x[k].l, w[k].h, fx_mad(x[k].h, w[k].l, c));
+        a = fx_mad(x[k].h, w[k].h, a);
+    }
+    return (a << 2) + (c >> 30);
 }
-// the same sum term by term
-struct FxSum {
-    int64_t c = 0x80000000ll, a = 0;
+// two terms of the last sum / 2^62, rounded: halves, because the small products of
+// all four terms could pass 2^63
+struct FxHalf {
+    int64_t c = 0x80000000ll >> 2, a = 0;
     __device__ __forceinline__ void add(Fx x, Fx w) {
         c = fx_mad(x.l, w.h, fx_mad(x.h, w.l, c));
         a = fx_mad(x.h, w.h, a);
     }
-    __device__ __forceinline__ int64_t get() const { return a + (c >> 32); }
+    __device__ __forceinline__ int64_t get() const { return (a << 2) + (c >> 30); }
 };
 
-// the row sum r 2^(e - 54) as a double
+// a row sum r 2^(e - 60) below 2^(e - 7)
+__device__ __forceinline__ bool fx_small(int64_t r) { return abs((int)(r >> 32)) < 1 << 21; }
+// |x| |w| in units of 2^(u + 2), x.h in units of 2^u (w.h: 2^-30)
+__device__ __forceinline__ uint32_t fx_abs_mul(uint32_t x, Fx w) { return __umulhi(x, (uint32_t)abs(w.h)); }
+// the sum of a row's central |w x| of one plane, in units of 2^(e - 22), from its four values
+__device__ __forceinline__ uint32_t fx_central(Fx x11, Fx x12, Fx x21, Fx x22, Fx wx, Fx wy1, Fx wy2, Fx wz1, Fx wz2) {
+    const uint32_t y1 = fx_abs_mul((uint32_t)abs(x11.h), wz1) + fx_abs_mul((uint32_t)abs(x12.h), wz2);
+    const uint32_t y2 = fx_abs_mul((uint32_t)abs(x21.h), wz1) + fx_abs_mul((uint32_t)abs(x22.h), wz2);
+    return fx_abs_mul(fx_abs_mul(y1, wy1) + fx_abs_mul(y2, wy2), wx);
+}
+// both planes' below 2^(e - 7)
+__device__ __forceinline__ bool fx_weak(uint32_t central) { return central < 1u << 15; }
+
+// the row sum r 2^(e - 60) as a double
 __device__ __forceinline__ double fx_to_double(int64_t r, uint32_t e20) {
-    return (double)r * __hiloint2double((int)(e20 - (54u << 20)), 0);
+    return (double)r * __hiloint2double((int)(e20 - (60u << 20)), 0);
 }
 
 // four consecutive weights

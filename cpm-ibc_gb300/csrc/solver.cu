@@ -566,16 +566,20 @@ __global__ void __launch_bounds__(128, EW_BPS) k_epass32w(OpView<float> op, cons
     e_ident32(op, warp, lane, act, x, t);
 }
 
-// a row that fixed point cannot hold, slot s of a K-wide batch
+// planes i0 .. i1 of a row in FP64, slot s of a K-wide batch: rows that fixed point
+// cannot hold, or not to the accuracy of this sum (fixed62.h)
 template <int K>
-__device__ __noinline__ double e_row_fp64(const double *__restrict__ w, const int32_t *__restrict__ gc, int s,
-                                          const double *__restrict__ x) {
+__device__ __noinline__ double e_row_fp64(const double *w, const int32_t *gc, int s, const double *x, int i0, int i1) {
     double acc = 0.0;
-    for (int i = 0; i < 4; ++i) {
-        double ay = 0.0;
+    for (int i = i0; i < i1; ++i) {
+        double xv[16], ay = 0.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) xv[q] = x[(int64_t)gc[16 * i + q] * K + s];
+#pragma unroll
         for (int j = 0; j < 4; ++j) {
             double az = 0.0;
-            for (int k = 0; k < 4; ++k) az += w[8 + k] * x[(int64_t)gc[16 * i + 4 * j + k] * K + s];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) az += w[8 + k] * xv[4 * j + k];
             ay += w[4 + j] * az;
         }
         acc += w[i] * ay;
@@ -631,7 +635,8 @@ __global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Sl
 #pragma unroll
             for (int q = 0; q < 32; ++q) v[q] = fx_from_double(xv[q], e20);
         }
-        const bool out = act && fx_out(e20), any_out = __any_sync(FULL, out);
+        const bool out = act && fx_out(e20);
+        uint32_t redo = out ? ~0u : 0u;  // rows of the group to sum in FP64; the last bit: any row from the 32nd on
         for (int c0 = p0; c0 < p1; c0 += EX_ROWS) {
             const int nr = min(p1 - c0, EX_ROWS);
             __syncwarp();
@@ -644,8 +649,7 @@ __global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Sl
                 Fx wy[4], wz[4];
                 fx_lds4(w + 4, wy);
                 fx_lds4(w + 8, wz);
-                FxSum sum;
-                if (h) sum.c = 0;  // the rounding bit once
+                FxHalf sum;
 #pragma unroll
                 for (int a = 0; a < 2; ++a) {
                     Fx ay[4];
@@ -657,27 +661,47 @@ __global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Sl
                     }
                     sum.add(fx_split(fx_dot4(ay, wy)), fx_lds1(w + 2 * h + a));
                 }
-                sum.c += __shfl_xor_sync(FULL, sum.c, 16);
-                sum.a += __shfl_xor_sync(FULL, sum.a, 16);
+                int64_t rv = sum.get();
+                rv += __shfl_xor_sync(FULL, rv, 16);
                 const int r = __shfl_sync(FULL, row, q), f = __shfl_sync(FULL, fl, q);
+                double acc = fx_to_double(rv, e20);
+                const bool small = act && !out && fx_small(rv);
+                if (__any_sync(FULL, small)) {
+                    // the centre's planes are 1 (h = 0, its second) and 2 (h = 1, its first)
+                    Fx uy[4], uz[4];
+                    fx_lds4(w + 4, uy);
+                    fx_lds4(w + 8, uz);
+                    uint32_t mid = fx_central(h ? v[5] : v[21], h ? v[6] : v[22], h ? v[9] : v[25], h ? v[10] : v[26],
+                                              fx_lds1(w + 1 + h), uy[1], uy[2], uz[1], uz[2]);
+                    mid += __shfl_xor_sync(FULL, mid, 16);
+                    if (small && fx_weak(mid)) redo |= 1u << min(c0 + q - p0, 31);
+                }
                 if (h == 0 && act && !out) {
-                    double acc = fx_to_double(sum.get(), e20);
                     if (f) acc = e_row_terms<double, 32>(op, (uint8_t)f, r, s, acc, x);
                     t[(uint32_t)r * 32u + s] = acc;
                 }
             }
         }
-        if (any_out) {  // these slots again, in FP64 (zeros stay zeros)
-            bool nz = false;
-            if (out)
+        const uint32_t any = __reduce_or_sync(FULL, redo);
+        if (any) {
+            bool nz = true;  // zeros stay zeros
+            if (out) {
+                nz = false;
                 for (int q = 0; q < 64; ++q) nz = nz || nonzero(xs[(uint32_t)op.gcols[64 * g + q] * 32u]);
-            for (int p = p0; p < p1; ++p)
-                if (out && h == 0) {
+            }
+            for (int p = p0; p < p1; ++p) {
+                const int bit = min(p - p0, 31);
+                if (!(any >> bit & 1)) continue;
+                const bool mine = redo >> bit & 1;
+                double acc = 0.0;
+                if (mine && nz) acc = e_row_fp64<32>(op.w_ord + 12 * (size_t)p, op.gcols + 64 * g, s, x, 2 * h, 2 * h + 2);
+                acc += __shfl_xor_sync(FULL, acc, 16);
+                if (mine && h == 0) {
                     const int r = op.ord[p], f = op.fl_ord[p] & F_TERMS;
-                    double acc = nz ? e_row_fp64<32>(op.w_ord + 12 * (size_t)p, op.gcols + 64 * g, s, x) : 0.0;
                     if (f) acc = e_row_terms<double, 32>(op, (uint8_t)f, r, s, acc, x);
                     t[(uint32_t)r * 32u + s] = acc;
                 }
+            }
         }
     }
     e_ident32(op, warp, lane, act32, x, t);
@@ -703,7 +727,8 @@ struct E1Group<double> {
     alignas(16) Fx x[66];
 };
 
-__device__ __forceinline__ float e1_row(const OpView<float> &op, int64_t p, uint32_t, const E1Group<float> &g) {
+// row p of a group; small: what it reads may outweigh its terms (e1_redo)
+__device__ __forceinline__ float e1_row(const OpView<float> &op, int64_t p, uint32_t, const E1Group<float> &g, bool &) {
     float w[12];
     load_w12(op.w_ord + 12 * p, w);
     float acc = 0.f;
@@ -724,12 +749,13 @@ __device__ __forceinline__ float e1_row(const OpView<float> &op, int64_t p, uint
     return acc;
 }
 
-__device__ __forceinline__ double e1_row(const OpView<double> &op, int64_t p, uint32_t e20, const E1Group<double> &g) {
+__device__ __forceinline__ double e1_row(const OpView<double> &op, int64_t p, uint32_t e20, const E1Group<double> &g, bool &small) {
     const int2 *w = op.w_fix + 12 * p;
-    Fx wx[4], wy[4], wz[4], ax[4];
+    Fx wx[4], wy[4], wz[4];
     fx_load4(w, wx);
     fx_load4(w + 4, wy);
     fx_load4(w + 8, wz);
+    FxHalf sum[2];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         Fx ay[4];
@@ -740,9 +766,58 @@ __device__ __forceinline__ double e1_row(const OpView<double> &op, int64_t p, ui
             const Fx v[4] = {Fx{a.x, a.y}, Fx{a.z, a.w}, Fx{b.x, b.y}, Fx{b.z, b.w}};
             ay[j] = fx_split(fx_dot4(v, wz));
         }
-        ax[i] = fx_split(fx_dot4(ay, wy));
+        sum[i >> 1].add(fx_split(fx_dot4(ay, wy)), wx[i]);
     }
-    return fx_to_double(fx_dot4(ax, wx), e20);
+    const int64_t r = sum[0].get() + sum[1].get();
+    small = fx_small(r);
+    return fx_to_double(r, e20);
+}
+
+// The rows of a warp's run that take the FP64 sum (fixed62.h), or acc for the
+// others.  How this lane's row stands: 1 if its sum is small and its central terms
+// decide, 2 if fixed point cannot hold it.  The groups' values are gathered again,
+// as they are, into the places of the aligned ones.  All lanes call.
+__device__ __noinline__ double e1_redo(int how, double acc, const int2 *wf, const double *wd, const int32_t *gc, int ng, int mine,
+                                       E1Group<double> *sh, const double *x, int lane) {
+    if (how == 1) {
+        Fx wx[4], wy[4], wz[4];
+        fx_load4(wf, wx);
+        fx_load4(wf + 4, wy);
+        fx_load4(wf + 8, wz);
+        const Fx *l = sh[mine].x + 16, *m = l + 16;
+        how = fx_weak(fx_central(l[5], l[6], l[9], l[10], wx[1], wy[1], wy[2], wz[1], wz[2]) +
+                      fx_central(m[5], m[6], m[9], m[10], wx[2], wy[1], wy[2], wz[1], wz[2])) ? 2 : 0;
+    }
+    if (!__any_sync(FULL, how == 2)) return acc;
+    __syncwarp();
+    for (int g = 0; g < ng; ++g)
+        if (__any_sync(FULL, how == 2 && mine == g)) {
+            const double a = x[gc[64 * g + lane]], b = x[gc[64 * g + lane + 32]];
+            double *v = (double *)sh[g].x;
+            v[lane] = a;
+            v[lane + 32] = b;
+        }
+    __syncwarp();
+    if (how == 2) {
+        double w[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k) w[k] = wd[k];
+        const double *v = (const double *)sh[mine].x;
+        acc = 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            double ay = 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                double az = 0.0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) az += w[8 + k] * v[16 * i + 4 * j + k];
+                ay += w[4 + j] * az;
+            }
+            acc += w[i] * ay;
+        }
+    }
+    return acc;
 }
 
 // one warp's run: the operator's tables of it
@@ -808,9 +883,14 @@ __device__ __forceinline__ void e1_run(const OpView<T> &op, const E1Run &q, int 
             }
     }
     __syncwarp();
-    T acc = e1_row(op, q.p, e20, sh[mine]);
-    if constexpr (sizeof(T) == 8)
-        if (fx_out(e20)) acc = zero ? 0.0 : e_row_fp64<1>(op.w_ord + 12 * q.p, op.gcols + 64 * (int64_t)(q.ch.x + mine), 0, x);
+    bool small = false;
+    T acc = e1_row(op, q.p, e20, sh[mine], small);
+    if constexpr (sizeof(T) == 8) {
+        const int how = lane >= nr ? 0 : fx_out(e20) ? (zero ? 0 : 2) : small ? 1 : 0;
+        if (zero) acc = 0.0;
+        if (__any_sync(FULL, how != 0))
+            acc = e1_redo(how, acc, op.w_fix + 12 * q.p, op.w_ord + 12 * q.p, op.gcols + 64 * (int64_t)q.ch.x, ng, mine, sh, x, lane);
+    }
     if (lane < nr) {
         if (q.fl) acc = e_row_terms<T, 1>(op, q.fl, q.r, 0, acc, x);
         t[q.r] = acc;
