@@ -855,7 +855,7 @@ __device__ __forceinline__ void e1_run(const OpView<T> &op, const E1Run &q, int 
         }
     const int mine = __popc((uint32_t)q.ch.z & (0xffffffffu >> (31 - lane))) - 1;  // the row's group
     uint32_t e20 = FX_EMIN;  // exponent field of the row's group
-    bool zero = false;       // the warp's groups of smallest exponent hold zeros only
+    bool zero = false;       // and holds zeros only
     __syncwarp();
     if constexpr (sizeof(T) == 8) {
 #pragma unroll
@@ -867,12 +867,12 @@ __device__ __forceinline__ void e1_run(const OpView<T> &op, const E1Run &q, int 
                 sh[g].x[lane + 32] = fx_from_double(xb[g], e);
             }
         if (__any_sync(FULL, e20 == 0)) {
-            bool nz = false;
 #pragma unroll
             for (int g = 0; g < E1_GROUPS; ++g)
-                if (g < ng) nz = nz || nonzero(xa[g]) || nonzero(xb[g]);
-            nz = __any_sync(FULL, nz);  // every lane votes
-            zero = e20 == 0 && !nz;
+                if (g < ng) {
+                    const bool nz = __any_sync(FULL, nonzero(xa[g]) || nonzero(xb[g]));  // every lane votes
+                    if (mine == g) zero = !nz;
+                }
         }
     } else {
 #pragma unroll
