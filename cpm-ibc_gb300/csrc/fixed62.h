@@ -35,6 +35,10 @@
 //
 // A stencil with an infinity, a NaN or only values below 2^-895 (nothing is
 // left of the exponent range to align to) takes the FP64 sum as well.
+//
+// E(-x) is -E(x) bit for bit, as in FP64, although truncation and rounding are not
+// symmetric here: a stencil is summed with the sign that makes one of its values
+// positive (flip: its centre, or the first that is not zero).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -60,25 +64,27 @@ __device__ __forceinline__ Fx fx_split(int64_t v) {
 }
 
 // the double (hi, lo) in units of 2^(e - 60), e the exponent of the field e20
-// (at least this value's own), truncated.  Zeros and subnormals come out as 0
-// or -1 (e is at least 128 above them).
-__device__ __forceinline__ Fx fx_from_double(uint32_t hi, uint32_t lo, uint32_t e20) {
+// (at least this value's own), truncated; negated where the high bit of flip is
+// set.  Zeros and subnormals come out as 0 or -1 (e is at least 128 above them).
+__device__ __forceinline__ Fx fx_from_double(uint32_t hi, uint32_t lo, uint32_t e20, uint32_t flip) {
     const uint32_t d = min((e20 - (hi & FX_EXP)) >> 20, 63u);
     const uint32_t mh = (hi & 0xfffffu) | 0x100000u;
     const uint64_t m = ((uint64_t)__funnelshift_l(lo, mh, 8) << 32) | (uint64_t)(lo << 8);
     const uint64_t v = m >> d;
-    const uint32_t s = (uint32_t)((int)hi >> 31);  // ones' complement of a negative value: one unit off
+    const uint32_t s = (uint32_t)((int)(hi ^ flip) >> 31);  // ones' complement of a negative value: one unit off
     return fx_split((int64_t)((((uint64_t)((uint32_t)(v >> 32) ^ s)) << 32) | (uint64_t)((uint32_t)v ^ s)));
 }
 
-// the double v in units of 2^(e - 59), 60 bits: six of them add up without overflow
-__device__ __forceinline__ int64_t fx60_from_double(double v, uint32_t e20) {
+// the double v in units of 2^(e - 59), 60 bits: six of them add up without overflow.
+// Ones' complement of a negative value: the caller counts them (sign: 0 or -1).
+__device__ __forceinline__ int64_t fx60_from_double(double v, uint32_t e20, int &sign) {
     const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
     const uint32_t d = min((e20 - (hi & FX_EXP)) >> 20, 63u);
     const uint32_t mh = (hi & 0xfffffu) | 0x100000u;
     const uint64_t m = ((uint64_t)__funnelshift_l(lo, mh, 7) << 32) | (uint64_t)(lo << 7);
     const uint64_t r = m >> d;
     const uint32_t s = (uint32_t)((int)hi >> 31);
+    sign = (int)s;
     return (int64_t)((((uint64_t)((uint32_t)(r >> 32) ^ s)) << 32) | (uint64_t)((uint32_t)r ^ s));
 }
 
@@ -122,7 +128,7 @@ __device__ __forceinline__ uint32_t fx_central(Fx x11, Fx x12, Fx x21, Fx x22, F
 // both planes' below 2^(e - 7)
 __device__ __forceinline__ bool fx_weak(uint32_t central) { return central < 1u << 15; }
 
-// the row sum r 2^(e - 60) as a double
+// the row sum r 2^(e - 60) as a double, negated where the high bit of e20 is set
 __device__ __forceinline__ double fx_to_double(int64_t r, uint32_t e20) {
     return (double)r * __hiloint2double((int)(e20 - (60u << 20)), 0);
 }

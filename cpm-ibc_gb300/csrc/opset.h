@@ -399,8 +399,14 @@ __device__ __forceinline__ double l_row(const LCoef &lc, double x, const double 
         return fma(lc.c1, off, cx);
     }
     int64_t v = 0;
+    int neg = 0;
 #pragma unroll
-    for (int d = 0; d < 6; ++d) v += fx60_from_double(t[d], e20);
+    for (int d = 0; d < 6; ++d) {
+        int s;
+        v += fx60_from_double(t[d], e20, s);
+        neg += s;
+    }
+    v -= neg;  // two's complement: equal values of opposite sign cancel, as they do in FP64
     const double c1 = __hiloint2double(__double2hiint(lc.c1) + (int)(e20 - (1082u << 20)), __double2loint(lc.c1));
     return fma(c1, (double)v, cx);
 }

@@ -589,8 +589,8 @@ __device__ __noinline__ double e_row_fp64(const double *w, const int32_t *gc, in
 
 __device__ __forceinline__ uint32_t exp_field(double v) { return (uint32_t)__double2hiint(v) & FX_EXP; }
 __device__ __forceinline__ bool nonzero(double v) { return ((uint32_t)__double2hiint(v) << 1 | (uint32_t)__double2loint(v)) != 0; }
-__device__ __forceinline__ Fx fx_from_double(double v, uint32_t e20) {
-    return fx_from_double((uint32_t)__double2hiint(v), (uint32_t)__double2loint(v), e20);
+__device__ __forceinline__ Fx fx_from_double(double v, uint32_t e20, uint32_t flip) {
+    return fx_from_double((uint32_t)__double2hiint(v), (uint32_t)__double2loint(v), e20, flip);
 }
 // nothing to align to (zeros, subnormals and values below 2^-895), or infinities and NaN
 __device__ __forceinline__ bool fx_out(uint32_t e20) { return e20 - FX_EMIN >= FX_EXP - FX_EMIN; }
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Sl
         const int64_t g = gl.g;
         const int p0 = op.grp[g], p1 = op.grp[g + 1];
         Fx v[32];
-        uint32_t e20 = 0;
+        uint32_t e20 = 0, flip;
         {
             double xv[32];
 #pragma unroll
@@ -632,8 +632,19 @@ __global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Sl
 #pragma unroll
             for (int q = 0; q < 32; ++q) e20 = max(e20, exp_field(xv[q]));
             e20 = max(e20, __shfl_xor_sync(FULL, e20, 16));
+            // the slot's sign: its centre's (plane 1, h = 0), else its first value's that is not zero
+            uint32_t mine = nonzero(xv[21]) ? (uint32_t)__double2hiint(xv[21]) | 1u : 0u;
+            flip = __shfl_sync(FULL, mine, lane & 15);
+            if (__any_sync(FULL, flip == 0 && e20 != 0)) {
 #pragma unroll
-            for (int q = 0; q < 32; ++q) v[q] = fx_from_double(xv[q], e20);
+                for (int q = 31; q >= 0; --q)
+                    if (nonzero(xv[q])) mine = (uint32_t)__double2hiint(xv[q]) | 1u;
+                const uint32_t a = __shfl_sync(FULL, mine, lane & 15), b = __shfl_sync(FULL, mine, lane | 16);
+                if (flip == 0) flip = a ? a : b;
+            }
+            flip &= 0x80000000u;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] = fx_from_double(xv[q], e20, flip);
         }
         const bool out = act && fx_out(e20);
         uint32_t redo = out ? ~0u : 0u;  // rows of the group to sum in FP64; the last bit: any row from the 32nd on
@@ -664,7 +675,7 @@ __global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Sl
                 int64_t rv = sum.get();
                 rv += __shfl_xor_sync(FULL, rv, 16);
                 const int r = __shfl_sync(FULL, row, q), f = __shfl_sync(FULL, fl, q);
-                double acc = fx_to_double(rv, e20);
+                double acc = fx_to_double(rv, e20 | flip);
                 const bool small = act && !out && fx_small(rv);
                 if (__any_sync(FULL, small)) {
                     // the centre's planes are 1 (h = 0, its second) and 2 (h = 1, its first)
@@ -854,7 +865,7 @@ __device__ __forceinline__ void e1_run(const OpView<T> &op, const E1Run &q, int 
             xb[g] = x[q.cb[g]];
         }
     const int mine = __popc((uint32_t)q.ch.z & (0xffffffffu >> (31 - lane))) - 1;  // the row's group
-    uint32_t e20 = FX_EMIN;  // exponent field of the row's group
+    uint32_t e20 = FX_EMIN, flip = 0;  // exponent field and sign of the row's group
     bool zero = false;       // and holds zeros only
     __syncwarp();
     if constexpr (sizeof(T) == 8) {
@@ -862,9 +873,21 @@ __device__ __forceinline__ void e1_run(const OpView<T> &op, const E1Run &q, int 
         for (int g = 0; g < E1_GROUPS; ++g)
             if (g < ng) {
                 const uint32_t e = __reduce_max_sync(FULL, max(exp_field(xa[g]), exp_field(xb[g])));
-                if (mine == g) e20 = e;
-                sh[g].x[lane] = fx_from_double(xa[g], e);
-                sh[g].x[lane + 32] = fx_from_double(xb[g], e);
+                // the group's sign: its centre's, else its first value's that is not zero
+                uint32_t f = __shfl_sync(FULL, (uint32_t)__double2hiint(xa[g]), 21);
+                if (f << 1 == 0) {  // the same in every lane
+                    const unsigned na = __ballot_sync(FULL, nonzero(xa[g])), nb = __ballot_sync(FULL, nonzero(xb[g]));
+                    const uint32_t sa = __shfl_sync(FULL, (uint32_t)__double2hiint(xa[g]), na ? __ffs(na) - 1 : 0);
+                    const uint32_t sb = __shfl_sync(FULL, (uint32_t)__double2hiint(xb[g]), nb ? __ffs(nb) - 1 : 0);
+                    f = na ? sa : nb ? sb : 0u;
+                }
+                f &= 0x80000000u;
+                if (mine == g) {
+                    e20 = e;
+                    flip = f;
+                }
+                sh[g].x[lane] = fx_from_double(xa[g], e, f);
+                sh[g].x[lane + 32] = fx_from_double(xb[g], e, f);
             }
         if (__any_sync(FULL, e20 == 0)) {
 #pragma unroll
@@ -884,7 +907,7 @@ __device__ __forceinline__ void e1_run(const OpView<T> &op, const E1Run &q, int 
     }
     __syncwarp();
     bool small = false;
-    T acc = e1_row(op, q.p, e20, sh[mine], small);
+    T acc = e1_row(op, q.p, e20 | flip, sh[mine], small);
     if constexpr (sizeof(T) == 8) {
         const int how = lane >= nr ? 0 : fx_out(e20) ? (zero ? 0 : 2) : small ? 1 : 0;
         if (zero) acc = 0.0;
