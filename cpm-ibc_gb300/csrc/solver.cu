@@ -2405,8 +2405,10 @@ static int solve_pass(cpm_solver_s *s, const SolveParams &P, const std::vector<c
     cudaGraphExec_t gexec = nullptr;
     const bool one_kernel = K == 1 && !P.mixed && s->plain1_G > 0;
     if (!one_kernel) CPM_TRY(prepare_graph<K>(s, P, &gexec));
-    const int chunk = one_kernel ? plain1_iters(P) : graph_chunk(s, P);
-    const int64_t max_chunks = (int64_t)P.max_iters / chunk + 2 * P.max_refine + 4;
+    // launches at most, by the graph's iterations either way: a restart ends a launch of
+    // k_plain1 early, and may do so after a few iterations
+    const int chunk = plain1_iters(P);
+    const int64_t max_chunks = (int64_t)P.max_iters / graph_chunk(s, P) + 2 * P.max_refine + 4;
     const long long per_graph = graph_launches(s, P);
     bool done = false;
     for (int64_t c = 0; c < max_chunks && !done; ++c) {
