@@ -2096,8 +2096,9 @@ struct cpm_solver_s {
     // captured iteration graphs (kernel arguments are fixed pointers; per-solve
     // parameters live in device memory, so a graph is reused while they match)
     cudaGraphExec_t g_plain = nullptr, g_mixed = nullptr;
-    // k_plain1's grid (0: this solver iterates by graphs), partial sums and barrier
-    int plain1_G = 0;
+    // k_plain1's grid (0: this solver iterates by graphs), partial sums and barrier;
+    // plain1_set: the grid set by hand (-1: the rule)
+    int plain1_G = 0, plain1_set = -1;
     DBuf<double> plain1_partial;
     DBuf<unsigned int> plain1_bar;
     SolveParams gp_plain{}, gp_mixed{};
@@ -2186,15 +2187,31 @@ static int plain1_blocks(const cpm_solver_s *s) {
     const int64_t most = runs <= sms * (BS / 32) ? sms : sms * std::min(per_sm, PLAIN1_BPS);
     return (int)std::min<int64_t>(most, std::max<int64_t>(runs, (s->D + BS - 1) / BS));
 }
-static int plain1_launch(cpm_solver_s *s, const SolveParams &P, int iters) {
+// the grid of s's one-kernel solves and what they need besides
+static int plain1_setup(cpm_solver_s *s) {
+    if (s->K != 1) return 0;
+    s->plain1_G = s->plain1_set >= 0 ? s->plain1_set : s->D <= PLAIN1_MAX_D ? plain1_blocks(s) : 0;
+    if (s->plain1_G == 0) return 0;
+    if (s->plain1_partial.n < 6 * (size_t)s->plain1_G) CPM_TRY(s->plain1_partial.alloc(6 * (size_t)s->plain1_G));
+    if (!s->plain1_bar.n) {
+        CPM_TRY(s->plain1_bar.alloc(2));
+        CPM_TRY(s->h_bar.alloc(1));
+    }
+    return 0;
+}
+static int plain1_launch(cpm_solver_s *s, const SolveParams &P, int iters, bool *refused) {
     cudaStream_t st = stream();
     Plain1 a{s->op->view<double>(), s->slots.p, P, s->m, s->n, P.precond == 2 ? JACOBI_OMEGA : 1.0,
              P.precond == 0 ? nullptr : s->pinv64.p, s->x64.p, s->dr.p, s->dr0.p, s->dp.p, s->dv.p, s->ds.p, s->dt.p, s->dy.p,
              s->dz.p, s->te64.p, s->plain1_partial.p, s->plain1_bar.p, iters};
     CPM_CUDA_TRY(cudaMemsetAsync(s->plain1_bar.p, 0, 2 * sizeof(unsigned int), st));
     void *args[] = {&a};
-    CPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_plain1, dim3(s->plain1_G), dim3(BS), args, 0, st));
-    count_launches(1);
+    // a context may hold fewer blocks at once than at the solver's creation
+    *refused = cudaLaunchCooperativeKernel((const void *)k_plain1, dim3(s->plain1_G), dim3(BS), args, 0, st) != cudaSuccess;
+    if (*refused)
+        cudaGetLastError();
+    else
+        count_launches(1);
     return 0;
 }
 
@@ -2403,7 +2420,7 @@ static int solve_pass(cpm_solver_s *s, const SolveParams &P, const std::vector<c
     }
     CPM_CUDA_TRY(cudaGetLastError());
     cudaGraphExec_t gexec = nullptr;
-    const bool one_kernel = K == 1 && !P.mixed && s->plain1_G > 0;
+    bool one_kernel = K == 1 && !P.mixed && s->plain1_G > 0;
     if (!one_kernel) CPM_TRY(prepare_graph<K>(s, P, &gexec));
     // launches at most, by the graph's iterations either way: a restart ends a launch of
     // k_plain1 early, and may do so after a few iterations
@@ -2413,9 +2430,17 @@ static int solve_pass(cpm_solver_s *s, const SolveParams &P, const std::vector<c
     bool done = false;
     for (int64_t c = 0; c < max_chunks && !done; ++c) {
         if (one_kernel) {
-            CPM_TRY(plain1_launch(s, P, chunk));
-            CPM_CUDA_TRY(cudaMemcpyAsync(&s->h_bar[0], s->plain1_bar.p + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-        } else {
+            bool refused;
+            CPM_TRY(plain1_launch(s, P, chunk, &refused));
+            if (refused) {  // the graph goes on from the same slot and vectors, here and from now on
+                s->plain1_G = 0;
+                one_kernel = false;
+                CPM_TRY(prepare_graph<K>(s, P, &gexec));
+            } else {
+                CPM_CUDA_TRY(cudaMemcpyAsync(&s->h_bar[0], s->plain1_bar.p + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+            }
+        }
+        if (!one_kernel) {
             CPM_CUDA_TRY(cudaGraphLaunch(gexec, st));
             count_launches(per_graph);
         }
@@ -2468,7 +2493,10 @@ static int run_solve(cpm_solver_s *s, int k, const cpm_solve_opts *o, cpm_solve_
     // a 32-slot FP64 iteration costs about 14 one-slot ones: a few right-hand sides
     // are solved again one at a time
     if (K == 32 && n_redo > 0 && n_redo < 14) {
-        if (!s->fb1) CPM_TRY(cpm_solver_create(s->op, s->m, s->n, 1, &s->fb1));
+        if (!s->fb1) {
+            CPM_TRY(cpm_solver_create(s->op, s->m, s->n, 1, &s->fb1));
+            CPM_TRY(cpm_solver_set_one_kernel(s->fb1, s->plain1_set));
+        }
         cpm_solve_opts o64 = *o;
         o64.precision = 0;
         const int64_t D = s->D;
@@ -2548,17 +2576,20 @@ extern "C" int cpm_solver_create(cpm_opset_t op, double m, double n, int32_t ksl
         return bail(rc);
     k_pinv<double><<<nblk(s->D), BS, 0, stream()>>>(op->view<double>(), m, n, s->pinv64.p);
     if (cudaGetLastError() != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "pinv kernel"));
-    if (s->K == 1 && s->D <= PLAIN1_MAX_D) {
-        s->plain1_G = plain1_blocks(s);
-        if ((rc = s->plain1_partial.alloc(6 * (size_t)std::max(1, s->plain1_G))) || (rc = s->plain1_bar.alloc(2)) ||
-            (rc = s->h_bar.alloc(1)))
-            return bail(rc);
-    }
+    if ((rc = plain1_setup(s))) return bail(rc);
     cudaEventCreate(&s->e0);
     cudaEventCreate(&s->e1);
     if (cudaStreamSynchronize(s->own) != cudaSuccess) return bail(fail(CPM_ERR_CUDA, "solver_create"));
     *out = s;
     return 0;
+}
+
+extern "C" int cpm_solver_set_one_kernel(cpm_solver_t s, int32_t blocks) {
+    if (!s || blocks < -1 || blocks > 65535) return fail(CPM_ERR_INVALID_ARG, "set_one_kernel: blocks must be in [-1, 65535]");
+    SolverScope sc(s);
+    s->plain1_set = blocks;
+    CPM_TRY(plain1_setup(s));
+    return s->fb1 ? cpm_solver_set_one_kernel(s->fb1, blocks) : 0;
 }
 
 extern "C" int cpm_solve_device(cpm_solver_t s, int32_t k, const void *b_dev, void *x_dev, const cpm_solve_opts *opts,

@@ -332,6 +332,14 @@ typedef struct cpm_solve_stats {
  * binds (m, n) to an operator set and allocates k slot columns of solver state. */
 int cpm_solver_create(cpm_opset_t op, double m, double n, int32_t kslots, cpm_solver_t *out);
 
+/* Launch shape of the solver's FP64 solves of one right-hand side (a 32-slot solver's
+ * own fallback solves among them): the thread blocks of the one kernel that iterates,
+ * 0 to iterate by graphs of kernels, -1 for the built-in choice by the number of rows.
+ * The kernel's blocks have to be on the device together; a launch of more is refused
+ * and the solver goes on by graphs.  Sums are grouped by block, so shapes change
+ * results within rounding.  No counterpart in the reference. */
+int cpm_solver_set_one_kernel(cpm_solver_t s, int32_t blocks);
+
 /* Solver::Solve (src/Solver.cpp:69-114) for k right-hand sides at once (k <= kslots);
  * b, x: host, RHS-major D*k.  stats: k entries (may be NULL). */
 int cpm_solve(cpm_solver_t s, int32_t k, const double *b, double *x, const cpm_solve_opts *opts, cpm_solve_stats *stats);
