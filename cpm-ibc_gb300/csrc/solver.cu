@@ -1685,6 +1685,7 @@ struct Plain1 {
     double *partial;     // the blocks' two sums, one place for each of an iteration's three reductions
     unsigned int *bar;   // arrivals, zero at launch; bar[1]: a wait ran out
     int iters;           // iterations at most
+    int polls;           // of a barrier's wait, then it gives up
 };
 
 // Barrier over the grid (a cooperative launch: every block is resident): 1.2 us
@@ -1692,7 +1693,7 @@ struct Plain1 {
 // and more: the readers hold up the writes.)  A wait that runs out, some seconds,
 // sets bar[1] and every block leaves: false.
 constexpr int PLAIN1_POLLS = 1 << 22;
-__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned &target) {
+__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned &target, int polls) {
     __shared__ bool met;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1700,7 +1701,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned &target
         // releases the block's writes, ordered before by the __syncthreads
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         bool ok = false;
-        for (int i = 0; i < PLAIN1_POLLS; ++i) {
+        for (int i = 0; i < polls; ++i) {
             unsigned now;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
             if ((int)(now - target) >= 0) {
@@ -1742,7 +1743,7 @@ __global__ void __launch_bounds__(BS, PLAIN1_BPS) k_plain1(Plain1 a) {
             partial[2 * blockIdx.x] = v[0];
             partial[2 * blockIdx.x + 1] = v[1];
         }
-        ok = grid_barrier(a.bar, target);
+        ok = grid_barrier(a.bar, target, a.polls);
         v[0] = v[1] = 0.0;
         for (unsigned b = tid; b < gridDim.x; b += BS) {
             v[0] += __ldcg(partial + 2 * b);
@@ -1772,7 +1773,7 @@ __global__ void __launch_bounds__(BS, PLAIN1_BPS) k_plain1(Plain1 a) {
             const int passes = a.P.precond == 2 ? a.P.sweeps : 1;
             for (int j = 1; j <= passes; ++j) {
                 // te = E~ y: every block's rows of y first, every row of te before it is read
-                if (!(ok = grid_barrier(a.bar, target))) return;
+                if (!(ok = grid_barrier(a.bar, target, a.polls))) return;
                 for (int64_t c = c0; c < op.n_chunk; c += warps) {
                     if (c != c0) e1_tables(op, c, lane, run);
                     e1_run(op, run, lane, eg[warp], (const double *)y, a.te);
@@ -1782,7 +1783,7 @@ __global__ void __launch_bounds__(BS, PLAIN1_BPS) k_plain1(Plain1 a) {
                     const int r = op.ident[k];
                     a.te[r] = y[r];
                 }
-                if (!(ok = grid_barrier(a.bar, target))) return;
+                if (!(ok = grid_barrier(a.bar, target, a.polls))) return;
                 const bool last = j == passes;
                 constexpr int UN = 2;
                 ROWS_UNR_N(D, UN) {
@@ -2097,8 +2098,8 @@ struct cpm_solver_s {
     // parameters live in device memory, so a graph is reused while they match)
     cudaGraphExec_t g_plain = nullptr, g_mixed = nullptr;
     // k_plain1's grid (0: this solver iterates by graphs), partial sums and barrier;
-    // plain1_set: the grid set by hand (-1: the rule)
-    int plain1_G = 0, plain1_set = -1;
+    // plain1_set, plain1_polls: the grid and the polls of a wait set by hand (-1: the rule)
+    int plain1_G = 0, plain1_set = -1, plain1_polls = -1;
     DBuf<double> plain1_partial;
     DBuf<unsigned int> plain1_bar;
     SolveParams gp_plain{}, gp_mixed{};
@@ -2203,7 +2204,8 @@ static int plain1_launch(cpm_solver_s *s, const SolveParams &P, int iters, bool 
     cudaStream_t st = stream();
     Plain1 a{s->op->view<double>(), s->slots.p, P, s->m, s->n, P.precond == 2 ? JACOBI_OMEGA : 1.0,
              P.precond == 0 ? nullptr : s->pinv64.p, s->x64.p, s->dr.p, s->dr0.p, s->dp.p, s->dv.p, s->ds.p, s->dt.p, s->dy.p,
-             s->dz.p, s->te64.p, s->plain1_partial.p, s->plain1_bar.p, iters};
+             s->dz.p, s->te64.p, s->plain1_partial.p, s->plain1_bar.p, iters,
+             s->plain1_polls >= 0 ? s->plain1_polls : PLAIN1_POLLS};
     CPM_CUDA_TRY(cudaMemsetAsync(s->plain1_bar.p, 0, 2 * sizeof(unsigned int), st));
     void *args[] = {&a};
     // a context may hold fewer blocks at once than at the solver's creation
@@ -2446,7 +2448,7 @@ static int solve_pass(cpm_solver_s *s, const SolveParams &P, const std::vector<c
         }
         CPM_CUDA_TRY(cudaMemcpyAsync(s->h_slots.data(), s->slots.p, sizeof(Slot) * K, cudaMemcpyDeviceToHost, st));
         CPM_CUDA_TRY(cudaStreamSynchronize(st));
-        if (one_kernel && s->h_bar[0]) return fail(CPM_ERR_TIMEOUT, "solve: a grid barrier ran out");
+        if (one_kernel && s->h_bar[0]) break;  // a barrier ran out: the slot stays unfinished (CPM_ERR_TIMEOUT)
         done = true;
         bool restart = false;
         for (int j = 0; j < K; ++j) {
@@ -2495,7 +2497,7 @@ static int run_solve(cpm_solver_s *s, int k, const cpm_solve_opts *o, cpm_solve_
     if (K == 32 && n_redo > 0 && n_redo < 14) {
         if (!s->fb1) {
             CPM_TRY(cpm_solver_create(s->op, s->m, s->n, 1, &s->fb1));
-            CPM_TRY(cpm_solver_set_one_kernel(s->fb1, s->plain1_set));
+            CPM_TRY(cpm_solver_set_one_kernel(s->fb1, s->plain1_set, s->plain1_polls));
         }
         cpm_solve_opts o64 = *o;
         o64.precision = 0;
@@ -2506,7 +2508,7 @@ static int run_solve(cpm_solver_s *s, int k, const cpm_solve_opts *o, cpm_solve_
             CPM_CUDA_TRY(cudaGetLastError());
             cpm_solve_stats s64;
             const int rc64 = cpm_solve_device(s->fb1, 1, s->fb1->b64.p, nullptr, &o64, &s64);
-            if (rc64 != 0 && rc64 != CPM_ERR_NOT_CONVERGED && rc64 != CPM_ERR_BREAKDOWN) return rc64;
+            if (rc64 != 0 && rc64 != CPM_ERR_NOT_CONVERGED && rc64 != CPM_ERR_BREAKDOWN && rc64 != CPM_ERR_TIMEOUT) return rc64;
             k_scatter_col<<<nblk(D), BS, 0, stream()>>>(D, 32, j, s->fb1->x64.p, s->x64.p);
             CPM_CUDA_TRY(cudaGetLastError());
             s64.iterations += st[j].iterations;
@@ -2584,12 +2586,14 @@ extern "C" int cpm_solver_create(cpm_opset_t op, double m, double n, int32_t ksl
     return 0;
 }
 
-extern "C" int cpm_solver_set_one_kernel(cpm_solver_t s, int32_t blocks) {
-    if (!s || blocks < -1 || blocks > 65535) return fail(CPM_ERR_INVALID_ARG, "set_one_kernel: blocks must be in [-1, 65535]");
+extern "C" int cpm_solver_set_one_kernel(cpm_solver_t s, int32_t blocks, int32_t wait_polls) {
+    if (!s || blocks < -1 || blocks > 65535 || wait_polls < -1 || wait_polls > PLAIN1_POLLS)
+        return fail(CPM_ERR_INVALID_ARG, "set_one_kernel: blocks must be in [-1, 65535], wait_polls in [-1, 4194304]");
     SolverScope sc(s);
     s->plain1_set = blocks;
+    s->plain1_polls = wait_polls;
     CPM_TRY(plain1_setup(s));
-    return s->fb1 ? cpm_solver_set_one_kernel(s->fb1, blocks) : 0;
+    return s->fb1 ? cpm_solver_set_one_kernel(s->fb1, blocks, wait_polls) : 0;
 }
 
 extern "C" int cpm_solve_device(cpm_solver_t s, int32_t k, const void *b_dev, void *x_dev, const cpm_solve_opts *opts,

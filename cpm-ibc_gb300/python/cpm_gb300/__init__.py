@@ -186,7 +186,7 @@ def lib():
         L.cpm_opset_autotune.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, P(TuneResult)]
         L.cpm_opset_set_launch.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]
         L.cpm_solver_create.argtypes = [vp, ctypes.c_double, ctypes.c_double, ctypes.c_int32, P(vp)]
-        L.cpm_solver_set_one_kernel.argtypes = [vp, ctypes.c_int32]
+        L.cpm_solver_set_one_kernel.argtypes = [vp, ctypes.c_int32, ctypes.c_int32]
         L.cpm_solve.argtypes = [vp, ctypes.c_int32, vp, vp, P(SolveOpts), P(SolveStats)]
         L.cpm_solve_device.argtypes = [vp, ctypes.c_int32, vp, vp, P(SolveOpts), P(SolveStats)]
         L.cpm_solver_destroy.argtypes = [vp]
@@ -564,9 +564,9 @@ class Solver:
         except Exception:
             pass
 
-    def set_one_kernel(self, blocks=-1):
+    def set_one_kernel(self, blocks=-1, wait_polls=-1):
         """launch shape of FP64 solves of one right-hand side (cpm_solver_set_one_kernel)"""
-        _check(lib().cpm_solver_set_one_kernel(self.h, blocks))
+        _check(lib().cpm_solver_set_one_kernel(self.h, blocks, wait_polls))
 
     def solve(self, b, tol=1e-10, precision=0, max_iters=100000, inner_tol=0.0, max_refine=400, raise_on_error=True,
               precond=DIAGONAL, precond_iters=0, refine_every=0):

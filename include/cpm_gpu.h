@@ -337,8 +337,12 @@ int cpm_solver_create(cpm_opset_t op, double m, double n, int32_t kslots, cpm_so
  * 0 to iterate by graphs of kernels, -1 for the built-in choice by the number of rows.
  * The kernel's blocks have to be on the device together; a launch of more is refused
  * and the solver goes on by graphs.  Sums are grouped by block, so shapes change
- * results within rounding.  No counterpart in the reference. */
-int cpm_solver_set_one_kernel(cpm_solver_t s, int32_t blocks);
+ * results within rounding.  wait_polls: how often a block looks for the others at a
+ * barrier before the kernel gives up, at most 4194304 (a few seconds, and the choice
+ * of -1); 0 gives up at once.  A solve that gave up reports CPM_ERR_TIMEOUT for that
+ * right-hand side, and its x is the unfinished iterate.  No counterpart in the
+ * reference. */
+int cpm_solver_set_one_kernel(cpm_solver_t s, int32_t blocks, int32_t wait_polls);
 
 /* Solver::Solve (src/Solver.cpp:69-114) for k right-hand sides at once (k <= kslots);
  * b, x: host, RHS-major D*k.  stats: k entries (may be NULL). */
