@@ -290,6 +290,7 @@ __device__ void cp_mesh_warp(const SurfaceParams &s, bool act, const double x[3]
     float above = CUDART_INF_F;  // the distance is at most this
     double best2 = 1e300, bestcp[3] = {0, 0, 0};
     int64_t bestp = -1;
+    int32_t tested[4] = {-1, -1, -1, -1};
     const int maxring = max(s.gn[0], max(s.gn[1], s.gn[2]));
     for (int ring = 0; ring <= maxring; ++ring) {
         const int a0 = max(lo[0] - ring, 0), a1 = min(hi[0] + ring, s.gn[0] - 1), b0 = max(lo[1] - ring, 0),
@@ -316,6 +317,12 @@ __device__ void cp_mesh_warp(const SurfaceParams &s, bool act, const double x[3]
                             }
                             const float far = above + slack + b.w;
                             if (!__any_sync(ALL, act && !(d2 > 1.00001f * (far * far)))) continue;
+                            // a large primitive is in many cells: not the last ones tested again
+                            if (p == tested[0] || p == tested[1] || p == tested[2] || p == tested[3]) continue;
+                            tested[3] = tested[2];
+                            tested[2] = tested[1];
+                            tested[1] = tested[0];
+                            tested[0] = p;
                             double q[3];
                             closest_on_prim(s, p, x, q);
                             const double dd[3] = {x[0] - q[0], x[1] - q[1], x[2] - q[2]}, q2 = dot3(dd, dd);
@@ -500,11 +507,12 @@ SurfaceParams SurfaceObj::params() const {
     return s;
 }
 
-// Cell-grid build for mesh primitives (counting pass + scatter pass on the device).
+// Cell-grid build for mesh primitives (counting pass + scatter pass on the device), a
+// warp per primitive: a large one is in tens of thousands of cells.
 __global__ void k_prim_cells(int tri, const double *__restrict__ v, const int32_t *__restrict__ prims, int64_t np, double lo0,
                              double lo1, double lo2, double h, int n0, int n1, int n2, int32_t *__restrict__ counts,
                              const int32_t *__restrict__ starts, int32_t *__restrict__ fill, int32_t *__restrict__ items) {
-    int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (p >= np) return;
     int nv = tri ? 3 : 2;
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
@@ -521,17 +529,17 @@ __global__ void k_prim_cells(int tri, const double *__restrict__ v, const int32_
         a[d] = max(0, min(n[d] - 1, (int)floor((lo[d] - g[d]) / h)));
         b[d] = max(0, min(n[d] - 1, (int)floor((hi[d] - g[d]) / h)));
     }
-    for (int i = a[0]; i <= b[0]; ++i)
-        for (int j = a[1]; j <= b[1]; ++j)
-            for (int k = a[2]; k <= b[2]; ++k) {
-                size_t c = ((size_t)i * n1 + j) * n2 + k;
-                if (!starts) {
-                    atomicAdd(&counts[c], 1);
-                } else {
-                    int slot = atomicAdd(&fill[c], 1);
-                    items[starts[c] + slot] = (int32_t)p;
-                }
-            }
+    const int64_t mj = b[1] - a[1] + 1, mk = b[2] - a[2] + 1, cells = (b[0] - a[0] + 1) * mj * mk;
+    for (int64_t e = threadIdx.x & 31; e < cells; e += 32) {
+        const int i = a[0] + (int)(e / (mj * mk)), j = a[1] + (int)(e / mk % mj), k = a[2] + (int)(e % mk);
+        const size_t c = ((size_t)i * n1 + j) * n2 + k;
+        if (!starts) {
+            atomicAdd(&counts[c], 1);
+        } else {
+            const int slot = atomicAdd(&fill[c], 1);
+            items[starts[c] + slot] = (int32_t)p;
+        }
+    }
 }
 
 // a sphere around each primitive: the vertices' mean, rounded to FP32, and the
@@ -610,7 +618,7 @@ int surface_init(SurfaceObj &s, const cpm_surface_desc *d, double cell_h) {
     unsigned nb = (unsigned)((d->nprims + bs - 1) / bs);
     CPM_TRY(s.mesh.sph.alloc((size_t)d->nprims));
     k_prim_spheres<<<nb, bs, 0, stream()>>>(tri, s.mesh.verts.p, s.mesh.prims.p, d->nprims, s.mesh.sph.p);
-    k_prim_cells<<<nb, bs, 0, stream()>>>(tri, s.mesh.verts.p, s.mesh.prims.p, d->nprims, s.mesh.glo[0], s.mesh.glo[1],
+    k_prim_cells<<<(unsigned)((32 * d->nprims + bs - 1) / bs), bs, 0, stream()>>>(tri, s.mesh.verts.p, s.mesh.prims.p, d->nprims, s.mesh.glo[0], s.mesh.glo[1],
                                           s.mesh.glo[2], h, s.mesh.gn[0], s.mesh.gn[1], s.mesh.gn[2], counts.p, nullptr,
                                           nullptr, nullptr);
     CPM_CUDA_TRY(cudaGetLastError());
@@ -621,7 +629,7 @@ int surface_init(SurfaceObj &s, const cpm_surface_desc *d, double cell_h) {
     CPM_TRY(s.mesh.cell_start.upload(start));
     CPM_TRY(s.mesh.cell_items.alloc(std::max<size_t>(1, (size_t)start[ncell])));
     CPM_TRY(counts.zero());
-    k_prim_cells<<<nb, bs, 0, stream()>>>(tri, s.mesh.verts.p, s.mesh.prims.p, d->nprims, s.mesh.glo[0], s.mesh.glo[1],
+    k_prim_cells<<<(unsigned)((32 * d->nprims + bs - 1) / bs), bs, 0, stream()>>>(tri, s.mesh.verts.p, s.mesh.prims.p, d->nprims, s.mesh.glo[0], s.mesh.glo[1],
                                           s.mesh.glo[2], h, s.mesh.gn[0], s.mesh.gn[1], s.mesh.gn[2], nullptr,
                                           s.mesh.cell_start.p, counts.p, s.mesh.cell_items.p);
     CPM_CUDA_TRY(cudaGetLastError());
@@ -666,11 +674,15 @@ __global__ void k_brick_candidates(SurfaceParams s, GridParams g, double thresh,
     flag[b] = (fabs(d) <= thresh) ? 1 : 0;
 }
 
-// The same for a mesh, warp per brick: a brick with a primitive whose sphere comes
-// within thresh of its centre.  Spheres hold their primitives, so no brick of the
-// exact test is left out; a few more may be in, whose nodes the band test then
-// drops.  The lanes share out the primitives of the cells around the centre (one
-// thread a brick took 11 ms for the 4,913 bricks of the mesh at dx 0.02).
+// The same for a mesh, warp per brick: a brick with a primitive within thresh of its
+// centre.  The lanes share out the primitives of the cells around the centre (one
+// thread a brick took 11 ms for the 4,913 bricks of the mesh at dx 0.02).  Spheres in
+// FP32 decide where they can: farther than thresh, or wholly within it; in between
+// the primitive itself is tested in FP64, so that a mesh of few large primitives has
+// the bricks along its faces and not all those inside its spheres (a tetrahedron's
+// tube at dx 0.012: 645 ms by spheres alone, 178 ms with this test, 36 ms with the
+// cells of a primitive counted by a warp and repeated tests left out as well; 140 ms
+// with one thread a brick and no spheres).
 __global__ void k_brick_candidates_mesh(SurfaceParams s, GridParams g, double thresh, int32_t *__restrict__ flag) {
     const int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -683,7 +695,8 @@ __global__ void k_brick_candidates_mesh(SurfaceParams s, GridParams g, double th
         hi[d] = (int)fmin(floor((x[d] + thresh - s.glo[d]) / s.gh) + 1.0, (double)(s.gn[d] - 1));
     }
     const float xf[3] = {(float)x[0], (float)x[1], (float)x[2]};
-    const float slack = 2e-7f * (fabsf(xf[0]) + fabsf(xf[1]) + fabsf(xf[2])) + (float)thresh * 1.00001f;
+    const float slack = 2e-7f * (fabsf(xf[0]) + fabsf(xf[1]) + fabsf(xf[2]));  // x's rounding to FP32
+    const float above = (float)thresh * 1.00001f + slack, below = (float)thresh * 0.99999f - slack;
     bool found = false;
     for (int i = lo[0]; i <= hi[0] && !found; ++i)
         for (int j = lo[1]; j <= hi[1] && !found; ++j) {
@@ -692,9 +705,18 @@ __global__ void k_brick_candidates_mesh(SurfaceParams s, GridParams g, double th
             const int32_t t1 = lo[2] <= hi[2] ? __ldg(s.cell_start + row + hi[2] + 1) : 0;
             bool near = false;
             for (int32_t t = (lo[2] <= hi[2] ? __ldg(s.cell_start + row + lo[2]) : 0) + lane; t < t1; t += 32) {
-                const float4 c = __ldg(s.sph + __ldg(s.cell_items + t));
-                const float e0 = xf[0] - c.x, e1 = xf[1] - c.y, e2 = xf[2] - c.z, far = slack + c.w;
-                near = near || !(e0 * e0 + e1 * e1 + e2 * e2 > 1.00001f * (far * far));
+                const int32_t p = __ldg(s.cell_items + t);
+                const float4 c = __ldg(s.sph + p);
+                const float e0 = xf[0] - c.x, e1 = xf[1] - c.y, e2 = xf[2] - c.z, d2 = e0 * e0 + e1 * e1 + e2 * e2;
+                const float far = above + c.w, in = below - c.w;
+                if (near || d2 > 1.00001f * (far * far)) continue;
+                near = in > 0.f && d2 < 0.99999f * (in * in);
+                if (!near) {
+                    double q[3];
+                    closest_on_prim(s, p, x, q);
+                    const double dd[3] = {x[0] - q[0], x[1] - q[1], x[2] - q[2]};
+                    near = sqrt(dot3(dd, dd)) <= thresh;
+                }
             }
             found = __any_sync(0xffffffffu, near);
         }
