@@ -1668,8 +1668,8 @@ __global__ void __launch_bounds__(BS, 4) k_restart(OpView<T> op, Slot *sl, T m, 
     }
 }
 
-// ---- BiCGStab for one FP64 vector in one kernel.  At these sizes (11 to 300
-// thousand rows) an iteration is seven kernels of 3 to 15 us, and with Jacobi
+// ---- BiCGStab for one FP64 vector in one kernel.  At these sizes (11 to 180
+// thousand rows, plain1_pays) an iteration is seven kernels of 3 to 15 us, and with Jacobi
 // sweeps thousands of 5 us, of which starting, reading the slot's phase and
 // draining take more than half; here the blocks of a cooperative launch stay and
 // meet at a barrier (1.3 us) wherever rows of other blocks are read, the
@@ -2174,9 +2174,22 @@ static void plain_iteration(cpm_solver_s *s, const SolveParams &P) {
                                                 s->partial.p, s->counter.p);
 }
 
-// rows up to which one kernel iterates (216 thousand: 65 us an iteration, 68 by
-// the graph's kernels; these are long enough above, and hold more warps)
-constexpr int64_t PLAIN1_MAX_D = 250000;
+// Whether one kernel iterates, or a graph's kernels: these fill the device with more
+// warps, and pay their starts and ends.  Us an iteration on the two-circle sphere,
+// graph / one kernel:
+//   thousand rows     15           39           96           120          176          201
+//   diagonal          36 / 33      47 / 36      58 / 51      58 / 56      65 / 63      73 / 74
+//   2 Jacobi sweeps   72 / 60      100 / 69     137 / 105    146 / 118    156 / 147    167 / 175
+//   5                 122 / 118    181 / 137    243 / 210    259 / 240    283 / 299    307 / 358
+//   20                370 / 403    588 / 456    740 / 723    785 / 806    862 / 976    1025 / 1231
+//   200               3388 / 3985  5767 / 4628  7505 / 7661  7626 / 8240  8610 / 10058 9467 / 12172
+// A graph of many sweeps also has to be captured once a solver: with 2000, 20 ms.  A
+// geodesic (new solvers each) takes 44 ms by one kernel and 64 by graphs on 6
+// thousand rows, 243 and 248 on 166 thousand.
+constexpr int64_t PLAIN1_MAX_D = 180000, PLAIN1_SWEEPS_MAX_D = 120000;
+static bool plain1_pays(int64_t D, const SolveParams &P) {
+    return D <= (P.precond == 2 && P.sweeps > 4 ? PLAIN1_SWEEPS_MAX_D : PLAIN1_MAX_D);
+}
 // one launch of k_plain1: iterations until the slot leaves PH_ITER, at most `iters`
 static int plain1_blocks(const cpm_solver_s *s) {
     int per_sm = 0;
@@ -2422,7 +2435,7 @@ static int solve_pass(cpm_solver_s *s, const SolveParams &P, const std::vector<c
     }
     CPM_CUDA_TRY(cudaGetLastError());
     cudaGraphExec_t gexec = nullptr;
-    bool one_kernel = K == 1 && !P.mixed && s->plain1_G > 0;
+    bool one_kernel = K == 1 && !P.mixed && s->plain1_G > 0 && (s->plain1_set > 0 || plain1_pays(s->D, P));
     if (!one_kernel) CPM_TRY(prepare_graph<K>(s, P, &gexec));
     // launches at most, by the graph's iterations either way: a restart ends a launch of
     // k_plain1 early, and may do so after a few iterations

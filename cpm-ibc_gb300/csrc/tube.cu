@@ -389,7 +389,13 @@ __global__ void k_closest_points(SurfaceParams s, int64_t n, const double *__res
 // the primitives of each ring of cells, or of the whole mesh, first to bound the
 // distance by the spheres, then to test those that can be nearer.  The same rings,
 // arithmetic and choice as cp_mesh.  Lane by lane 6,700 projections took 2.4 ms.
-constexpr int64_t FEW_POINTS = 32768;  // a warp each; more are searched 32 to a warp
+// A call of cpm_closest_points within 0.1 of a surface, a warp per point / 32 points
+// to a warp: 20,480 triangles, 2 thousand points 1.1 / 3.4 ms, 8 thousand 1.4 / 3.5,
+// 33 thousand 2.8 / 4.1, 131 thousand 8.5 / 9.8, 262 thousand 16.3 / 16.2; 374
+// segments, 2 thousand 0.41 / 0.46, 8 thousand 0.53 / 0.48, 33 thousand 0.89 / 0.59
+// (scattered 0.87 / 0.81), 131 thousand 2.3 / 1.1.  The line lies where the triangles'
+// gain and the segments' loss are small.
+constexpr int64_t FEW_POINTS = 32768;
 __global__ void __launch_bounds__(128) k_closest_points_few(SurfaceParams s, int64_t n, const double *__restrict__ xs,
                                                             double *__restrict__ cp, double *__restrict__ dist, double max_dist) {
     constexpr unsigned ALL = 0xffffffffu;
