@@ -2482,6 +2482,31 @@ static int solve_pass(cpm_solver_s *s, const SolveParams &P, const std::vector<c
     return 0;
 }
 
+}  // namespace cpm
+
+// What 32 at once cost in units of one alone, fitted to within 15 % to runs on spheres
+// with two circles (measured, by thousand rows):
+//   rows              15    23    39    66    107   156   216   259   322   762
+//   FP64 iteration    4.7   6.2   7.1   8.9   10.2  13.0  14.5  16.2  16.3  21.6
+//   FP32 with FP64    2.7   3.3   2.8   3.0   3.3   3.7   3.9   4.3   4.4   4.8
+// and, by thousand tube nodes, on geodesics (the last on the torus at dx 0.01):
+//   nodes             6     11    22    42    85    166   260   1300
+//   32 sources        9.5   8.8   9.0   10.6  11.1  13.8  18.8  31.7
+// One vector is bound by latencies on small surfaces, 32 seldom, so one ratio for all
+// (15, 4.4 and 32, of the last but two columns) kept small surfaces from batches that
+// pay three times over.
+extern "C" double cpm_batch_cost(int64_t rows, int32_t kind) {
+    const double n = (double)std::max<int64_t>(1, rows);
+    switch (kind) {
+        case CPM_BATCH_FP64: return std::max(1.0, 14.45 * std::pow(n / 215662, 0.417));
+        case CPM_BATCH_MIXED: return std::max(1.0, 3.9 * std::pow(n / 215662, 0.14));
+        case CPM_BATCH_GEODESIC: return std::max(9.0, 15.5 * std::pow(n / 166390, 0.34));
+        default: return 0.0;
+    }
+}
+
+namespace cpm {
+
 // Solve k right-hand sides.  A mixed-precision slot that does not converge
 // (an FP32 inner iteration that cannot follow an ill-conditioned system, where
 // cond * 2^-24 ~ 1) is solved again by the plain FP64 path from x = 0; its
@@ -2505,9 +2530,9 @@ static int run_solve(cpm_solver_s *s, int k, const cpm_solve_opts *o, cpm_solve_
     }
     int n_redo = 0;
     for (int j = 0; j < k; ++j) n_redo += redo[j];
-    // a 32-slot FP64 iteration costs about 14 one-slot ones: a few right-hand sides
-    // are solved again one at a time
-    if (K == 32 && n_redo > 0 && n_redo < 14) {
+    // fewer right-hand sides than a 32-slot FP64 iteration costs one-slot ones are solved
+    // again one at a time
+    if (K == 32 && n_redo > 0 && n_redo < cpm_batch_cost(s->D, CPM_BATCH_FP64)) {
         if (!s->fb1) {
             CPM_TRY(cpm_solver_create(s->op, s->m, s->n, 1, &s->fb1));
             CPM_TRY(cpm_solver_set_one_kernel(s->fb1, s->plain1_set, s->plain1_polls));

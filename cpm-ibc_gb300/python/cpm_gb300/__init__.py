@@ -186,6 +186,8 @@ def lib():
         L.cpm_opset_autotune.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, P(TuneResult)]
         L.cpm_opset_set_launch.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]
         L.cpm_solver_create.argtypes = [vp, ctypes.c_double, ctypes.c_double, ctypes.c_int32, P(vp)]
+        L.cpm_batch_cost.argtypes = [ctypes.c_int64, ctypes.c_int32]
+        L.cpm_batch_cost.restype = ctypes.c_double
         L.cpm_solver_set_one_kernel.argtypes = [vp, ctypes.c_int32, ctypes.c_int32]
         L.cpm_solve.argtypes = [vp, ctypes.c_int32, vp, vp, P(SolveOpts), P(SolveStats)]
         L.cpm_solve_device.argtypes = [vp, ctypes.c_int32, vp, vp, P(SolveOpts), P(SolveStats)]
@@ -545,6 +547,14 @@ def sync():
 
 # preconditioners (src/Defines.h:13-18)
 IDENTITY, DIAGONAL, JACOBI = 0, 1, 2
+
+
+BATCH_FP64, BATCH_MIXED, BATCH_GEODESIC = 0, 1, 2
+
+
+def batch_cost(rows, kind):
+    """what 32 right-hand sides (or geodesics) at once cost in units of one alone (cpm_batch_cost)"""
+    return lib().cpm_batch_cost(int(rows), kind)
 
 
 class Solver:

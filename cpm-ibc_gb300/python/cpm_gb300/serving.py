@@ -10,9 +10,9 @@ fixed IBC curves) on the device.  Requests arrive over time:
   FP64 reliable updates; slots refill as solves finish);
 * ``geodesic``: heat-method distance from a tube node
   (GeodesicDistance::ComputeDistance, problems/GeodesicDistance.cpp:11-69),
-  which carries its own point-IBC operator and runs as one pipeline; once
-  GEO_BATCH_MIN geodesics wait on one surface they run together (up to 32) as one
-  batch on a slot-patched operator.
+  which carries its own point-IBC operator and runs as one pipeline; once as many
+  wait on one surface as a 32-source batch costs there (batch_cost) they run
+  together (up to 32) as one batch on a slot-patched operator.
 
 A surface's server is admitted only while the device has room for it (its
 estimated bytes within the HBM budget); an idle server is released to make
@@ -21,9 +21,9 @@ room for another surface's.
 A 32-slot batch costs about the same whether it holds one request or 32, so
 requests are solved alone by the plain FP64 path (the reference's algorithm,
 one right-hand side) while a surface's server is idle and fewer of them wait
-than the break-even count: a 32-slot iteration costs about K32_MIXED (FP32
-with FP64 reliable updates) or K32_FP64 one-RHS FP64 iterations, times the
-surface's measured ratio of mixed to FP64 iteration counts.  A surface's first
+than the break-even count: the cost of a 32-slot iteration (FP32 with FP64
+reliable updates, or FP64) in one-RHS FP64 iterations at the surface's number of
+rows (batch_cost), times its measured ratio of mixed to FP64 iteration counts.  A surface's first
 request is always solved alone, which measures its FP64 iteration count; its
 mixed-precision server then stops a solve after 6x that many iterations (and
 re-solves it in FP64).  The first mixed batch is a probe of PROBE requests
@@ -39,22 +39,21 @@ import time
 
 import numpy as np
 
-from . import DIAGONAL, Geodesic, GeodesicBatch, OpSet, Server, Solver, device_info
+from . import (BATCH_FP64, BATCH_GEODESIC, BATCH_MIXED, DIAGONAL, Geodesic, GeodesicBatch, OpSet, Server, Solver,
+               batch_cost, device_info)
 
 MAX_SLOTS = 32
 PROBE = 2  # requests in a surface's first mixed-precision batch
-K32_MIXED = 4.4  # 32-slot FP32 iteration (reliable updates amortised) / one-RHS FP64 iteration: 285 us / 65 us on
-# the two-circle sphere at dx 0.025
-K32_FP64 = 15.0  # 32-slot FP64 iteration / one-RHS FP64 iteration: 988 us / 65 us
-# geodesics waiting on one surface from which a batch beats solving them one by one: the
-# 32-source batch costs the same with 2 or 32 sources (FP64, lane = source), 50.1 s on the
-# torus at dx 0.01 against 1.58 s for one source alone
-GEO_BATCH_MIN = 32
+K32_MIXED, K32_FP64, GEO_BATCH_MIN = 4.4, 15.0, MAX_SLOTS  # batch costs of a surface of unknown size (some 300 thousand rows)
 
 
 class ServedSurface:
     """A device-resident surface: its tube, operator (with IBC curves) and, while
     admitted, its server."""
+
+    # costs of 32 at once in units of one alone: an FP32 and an FP64 iteration, and the
+    # geodesics waiting from which a batch beats one by one
+    k32_mixed, k32_fp64, geo_batch_min = K32_MIXED, K32_FP64, GEO_BATCH_MIN
 
     def __init__(self, name, tube, ibcs, m=0.0, n=-1.0, tol=1e-10, autotune=True):
         self.name, self.tube = name, tube
@@ -62,6 +61,9 @@ class ServedSurface:
         # launch shapes of this surface's E passes, timed once and kept with the operator
         self.tuning = self.opset.autotune(reps=10, fp64=True) if autotune else None
         self.rows = self.opset.rows()
+        self.k32_mixed = batch_cost(self.opset.D, BATCH_MIXED)
+        self.k32_fp64 = batch_cost(self.opset.D, BATCH_FP64)
+        self.geo_batch_min = min(MAX_SLOTS, int(np.ceil(batch_cost(tube.N, BATCH_GEODESIC))))
         self.n_ibc = len(ibcs)
         self.m, self.n, self.tol = m, n, tol
         self.server = None
@@ -86,9 +88,9 @@ class ServedSurface:
         if self.fp64_iters is None:
             return None
         if self.precision == 0:
-            return max(2, int(np.ceil(K32_FP64)))
+            return max(2, int(np.ceil(self.k32_fp64)))
         ratio = self.mixed_iters / self.fp64_iters if self.mixed_iters else 2.0
-        return max(2, int(np.ceil(K32_MIXED * ratio)))
+        return max(2, int(np.ceil(self.k32_mixed * ratio)))
 
     def rhs(self, values):
         """PoissonWithIBC::GetRHS with f = 0: Dirichlet value values[c] on curve c."""
@@ -107,10 +109,12 @@ class ServingLoop:
     """Serves a stream of requests over ServedSurfaces.
 
     hbm_budget: bytes the servers may hold together (default: the device's free
-    memory when the loop is created, less ``reserve`` bytes)."""
+    memory when the loop is created, less ``reserve`` bytes).
+    geodesic_batch_min: geodesics waiting on one surface that run as a batch
+    (default: each surface's own break-even)."""
 
     def __init__(self, surfaces, hbm_budget=None, reserve=1 << 30, geodesic_precision=1, dt_scale=1.0,
-                 geodesic_batch_min=GEO_BATCH_MIN):
+                 geodesic_batch_min=None):
         self.surfaces = {s.name: s for s in surfaces}
         self.geodesic_batch_min = geodesic_batch_min
         if hbm_budget is None:
@@ -238,17 +242,18 @@ class ServingLoop:
             _, _, name, what = min(cands)
             if what == "geodesic":
                 name0 = geo_wait[0]["surface"]
-                take = self._geo_take([r for r in geo_wait if r["surface"] == name0])
+                take = self._geo_take(self.surfaces[name0], [r for r in geo_wait if r["surface"] == name0])
                 geo_wait = [r for r in geo_wait if r not in take]
                 self._geodesics(self.surfaces[name0], take, keep_solutions, t0, out)
                 continue
             self._unit(self.surfaces[name], what, keep_solutions, t0, out)
         return out
 
-    def _geo_take(self, waiting):
-        """the geodesics to run next from those waiting on one surface (oldest first): up
-        to 32 as one batch once geodesic_batch_min wait, else the oldest alone"""
-        return waiting[:MAX_SLOTS] if len(waiting) >= self.geodesic_batch_min else waiting[:1]
+    def _geo_take(self, s, waiting):
+        """the geodesics to run next from those waiting on surface s (oldest first): up
+        to 32 as one batch once enough wait, else the oldest alone"""
+        least = s.geo_batch_min if self.geodesic_batch_min is None else self.geodesic_batch_min
+        return waiting[:MAX_SLOTS] if len(waiting) >= least else waiting[:1]
 
     def _geodesics(self, s, batch, keep_solutions, t0, out):
         """the waiting geodesics of surface s: one alone (its own point-IBC operator), two or
@@ -380,7 +385,7 @@ class ServingLoop:
                             geo.append(r)
                     c = self._candidate(s, now)
                     if geo and (c is None or geo[0]["t"] < c[0]):
-                        take = self._geo_take(geo)
+                        take = self._geo_take(s, geo)
                         geo = geo[len(take):]
                         self._geodesics(s, take, keep_solutions, t0, out)
                         continue

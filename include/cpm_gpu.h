@@ -344,6 +344,15 @@ int cpm_solver_create(cpm_opset_t op, double m, double n, int32_t kslots, cpm_so
  * reference. */
 int cpm_solver_set_one_kernel(cpm_solver_t s, int32_t blocks, int32_t wait_polls);
 
+/* What 32 right-hand sides at once cost in units of one alone, on an operator of that
+ * many rows: an iteration of FP64 solves, an FP32 iteration with its share of FP64
+ * updates against a one-slot FP64 one, a geodesic batch (rows: tube nodes).  From
+ * measurements on this GPU; decides when a mixed batch's fallback solves run as a
+ * batch, and serves callers that choose between one by one and a batch.  0 for
+ * another kind.  No counterpart in the reference. */
+enum { CPM_BATCH_FP64 = 0, CPM_BATCH_MIXED = 1, CPM_BATCH_GEODESIC = 2 };
+double cpm_batch_cost(int64_t rows, int32_t kind);
+
 /* Solver::Solve (src/Solver.cpp:69-114) for k right-hand sides at once (k <= kslots);
  * b, x: host, RHS-major D*k.  stats: k entries (may be NULL). */
 int cpm_solve(cpm_solver_t s, int32_t k, const double *b, double *x, const cpm_solve_opts *opts, cpm_solve_stats *stats);
