@@ -129,14 +129,6 @@ __device__ __forceinline__ int corner_node(const Corner &c, int l) {
 
 __device__ __forceinline__ Corner csel(bool p, const Corner &a, const Corner &b) { return p ? b : a; }
 
-// a[i] for a runtime i in 0..3 without a dynamically indexed (local-memory) array
-template <class T>
-__device__ __forceinline__ T pick4(const T (&a)[4], int i) {
-    const T lo = (i & 1) ? a[1] : a[0];
-    const T hi = (i & 1) ? a[3] : a[2];
-    return (i & 2) ? hi : lo;
-}
-
 // Thread-per-row gather: corners held in registers and picked with selects
 // (no dynamically indexed register arrays, so nothing spills to local memory).
 template <class T, int K>
@@ -257,7 +249,7 @@ __device__ __forceinline__ T e_row(const OpView<T> &op, int64_t r, int s, const 
     return acc;
 }
 
-// the 12 tricubic weights of a row (48 or 96 bytes, 16-byte aligned) as vectors
+// the 12 tricubic weights of a row (48 bytes, 16-byte aligned) as vectors
 __device__ __forceinline__ void load_w12(const float *w, float (&o)[12]) {
     const float4 *v = (const float4 *)w;
 #pragma unroll
@@ -267,15 +259,6 @@ __device__ __forceinline__ void load_w12(const float *w, float (&o)[12]) {
         o[4 * q + 1] = a.y;
         o[4 * q + 2] = a.z;
         o[4 * q + 3] = a.w;
-    }
-}
-__device__ __forceinline__ void load_w12(const double *w, double (&o)[12]) {
-    const double2 *v = (const double2 *)w;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        double2 a = __ldg(v + q);
-        o[2 * q] = a.x;
-        o[2 * q + 1] = a.y;
     }
 }
 
@@ -316,12 +299,6 @@ __device__ __forceinline__ uint64_t f2_sub(uint64_t a, uint64_t b) {
     return d;
 }
 
-// round-to-nearest fma and difference, never re-associated by the compiler
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-
 // four consecutive values from 16-byte aligned shared memory, as vector loads
 __device__ __forceinline__ void lds4(const float *p, float (&o)[4]) {
     const float4 v = *(const float4 *)p;
@@ -329,13 +306,6 @@ __device__ __forceinline__ void lds4(const float *p, float (&o)[4]) {
     o[1] = v.y;
     o[2] = v.z;
     o[3] = v.w;
-}
-__device__ __forceinline__ void lds4(const double *p, double (&o)[4]) {
-    const double2 a = *(const double2 *)p, b = *(const double2 *)(p + 2);
-    o[0] = a.x;
-    o[1] = a.y;
-    o[2] = b.x;
-    o[3] = b.y;
 }
 
 // the 16 columns of plane `plane` of group g: four 16-byte loads every lane makes alike

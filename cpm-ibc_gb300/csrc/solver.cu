@@ -5,8 +5,9 @@
 //        with the BiCGStab dot products fused into the L pass epilogue
 //   K10  vector updates of BiCGStab::Solve (src/BiCGStab.h:41-103) fused with
 //        their reductions; per-slot scalars stay on the device; reductions are
-//        accumulated in FP64 with a fixed-order two-level tree (deterministic
-//        and independent of the other slots' contents)
+//        accumulated in FP64 in a fixed order, in two levels of blocks for 32
+//        slots and one for one (deterministic and independent of the other
+//        slots' contents)
 //   K11  mixed precision: the Krylov iteration runs in FP32 (FP32 weights and
 //        vectors, FP64 reductions) and is refined in FP64 by reliable updates
 //        (Sleijpen & van der Vorst, "Reliable updated residuals in hybrid Bi-CG
@@ -1005,7 +1006,7 @@ static inline int default_bps(int64_t n) {
 
 // kernels one E pass of x launches
 template <class T, int K>
-static inline int epass_kernels(const OpView<T> &op, const T *) {
+static inline int epass_kernels(const OpView<T> &op) {
     return (K == 32 && op.n_sp_rows > 0) ? 2 : 1;
 }
 
@@ -1042,7 +1043,7 @@ int epass64_batch(const cpm_opset_s *o, bool slot_patches, const double *x, doub
         v.n_sp_rows = 0;
     }
     launch_epass<double, 32>(v, nullptr, -1, x, t, stream());
-    count_launches(epass_kernels<double, 32>(v, x));
+    count_launches(epass_kernels<double, 32>(v));
     CPM_CUDA_TRY(cudaGetLastError());
     return 0;
 }
@@ -1672,7 +1673,7 @@ __global__ void __launch_bounds__(BS, 4) k_restart(OpView<T> op, Slot *sl, T m, 
 // thousand rows, plain1_pays) an iteration is seven kernels of 3 to 15 us, and with Jacobi
 // sweeps thousands of 5 us, of which starting, reading the slot's phase and
 // draining take more than half; here the blocks of a cooperative launch stay and
-// meet at a barrier (1.3 us) wherever rows of other blocks are read, the
+// meet at a barrier (1.2 to 1.5 us) wherever rows of other blocks are read, the
 // operator's tables of a warp's first run stay in registers, and a solve stops at
 // the iteration that converges instead of the end of a graph.
 struct Plain1 {
@@ -2384,8 +2385,8 @@ static inline long long graph_launches(const cpm_solver_s *s, const SolveParams 
     const int chunk = graph_chunk(s, P);
     // an iteration: 5 vector / L-pass kernels and two E passes; a Jacobi sweep: an E
     // pass and the sweep; a reliable update: 4 kernels and an FP64 E pass
-    const long long e32 = s->K == 32 ? epass_kernels<float, 32>(s->op->view<float>(), s->fy.p) : 1;
-    const long long e64 = s->K == 32 ? epass_kernels<double, 32>(s->op->view<double>(), s->x64.p) : 1;
+    const long long e32 = s->K == 32 ? epass_kernels<float, 32>(s->op->view<float>()) : 1;
+    const long long e64 = s->K == 32 ? epass_kernels<double, 32>(s->op->view<double>()) : 1;
     const long long eit = P.mixed ? e32 : e64;
     return (5LL + 2 * eit + (P.precond == 2 ? 2LL * (P.sweeps - 1) * (e64 + 1) : 0)) * chunk +
            (P.mixed ? (4LL + e64) * (chunk / P.refine_every) : 0);
@@ -3145,8 +3146,8 @@ extern "C" int cpm_apply_device(cpm_opset_t op, double m, double n, int32_t kslo
             launch_after(k_lpass<double, 32>, row_grid(D, 32), BS, st, v, m, n, x, t, y);
         }
     }
-    count_launches(1 + (kslots == 32 ? (fp32 ? epass_kernels<float, 32>(op->view<float>(), (const float *)x_dev)
-                                              : epass_kernels<double, 32>(op->view<double>(), (const double *)x_dev))
+    count_launches(1 + (kslots == 32 ? (fp32 ? epass_kernels<float, 32>(op->view<float>())
+                                              : epass_kernels<double, 32>(op->view<double>()))
                                       : 1));
     CPM_CUDA_TRY(cudaGetLastError());
     return 0;
@@ -3209,7 +3210,6 @@ extern "C" int cpm_opset_autotune(cpm_opset_t op, int32_t reps, int32_t with_fp6
     CPM_CUDA_TRY(cudaGetLastError());
     cpm_tune_result res;
     memset(&res, 0, sizeof(res));
-    const int sms = sm_count();
     const int e32c[] = {8, 16, 24, 32, 48, 64, 96, 128}, pc[] = {4, 8, 16, 32, 64, 128}, e64c[] = {4, 8, 16, 32, 64};
     const OpView<float> v32 = op->view<float>();
     auto pick = [&](const int *c, int nc, int dflt, auto launch_with, float &best_us, float &dflt_us, int32_t &best) {
@@ -3335,8 +3335,8 @@ extern "C" int cpm_apply_device_noalloc(cpm_opset_t op, double m, double n, int3
             launch_after(k_lpass<double, 32>, row_grid(D, 32), BS, st, v, m, n, x, tt, y);
         }
     }
-    count_launches(1 + (kslots == 32 ? (fp32 ? epass_kernels<float, 32>(op->view<float>(), (const float *)x_dev)
-                                              : epass_kernels<double, 32>(op->view<double>(), (const double *)x_dev))
+    count_launches(1 + (kslots == 32 ? (fp32 ? epass_kernels<float, 32>(op->view<float>())
+                                              : epass_kernels<double, 32>(op->view<double>()))
                                       : 1));
     CPM_CUDA_TRY(cudaGetLastError());
     return 0;
