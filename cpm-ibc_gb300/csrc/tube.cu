@@ -520,24 +520,22 @@ __global__ void k_prim_cells(int tri, const double *__restrict__ v, const int32_
                              const int32_t *__restrict__ starts, int32_t *__restrict__ fill, int32_t *__restrict__ items) {
     const int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (p >= np) return;
-    int nv = tri ? 3 : 2;
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (int k = 0; k < nv; ++k) {
-        const double *q = v + 3 * prims[nv * p + k];
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = fmin(lo[d], q[d]);
-            hi[d] = fmax(hi[d], q[d]);
-        }
+    // lanes 0 .. 2: the first cell along each axis, 3 .. 5: the last
+    const int nv = tri ? 3 : 2, lane = threadIdx.x & 31, d = lane % 3;
+    double m = v[3 * prims[nv * p] + d];
+    for (int k = 1; k < nv; ++k) {
+        const double q = v[3 * prims[nv * p + k] + d];
+        m = lane < 3 ? fmin(m, q) : fmax(m, q);
     }
-    double g[3] = {lo0, lo1, lo2};
-    int n[3] = {n0, n1, n2}, a[3], b[3];
-    for (int d = 0; d < 3; ++d) {
-        a[d] = max(0, min(n[d] - 1, (int)floor((lo[d] - g[d]) / h)));
-        b[d] = max(0, min(n[d] - 1, (int)floor((hi[d] - g[d]) / h)));
+    const int cell = max(0, min((d == 0 ? n0 : d == 1 ? n1 : n2) - 1, (int)floor((m - (d == 0 ? lo0 : d == 1 ? lo1 : lo2)) / h)));
+    int a[3], b[3];
+    for (int e = 0; e < 3; ++e) {
+        a[e] = __shfl_sync(0xffffffffu, cell, e);
+        b[e] = __shfl_sync(0xffffffffu, cell, 3 + e);
     }
-    const int64_t mj = b[1] - a[1] + 1, mk = b[2] - a[2] + 1, cells = (b[0] - a[0] + 1) * mj * mk;
-    for (int64_t e = threadIdx.x & 31; e < cells; e += 32) {
-        const int i = a[0] + (int)(e / (mj * mk)), j = a[1] + (int)(e / mk % mj), k = a[2] + (int)(e % mk);
+    const int mj = b[1] - a[1] + 1, mk = b[2] - a[2] + 1, cells = (b[0] - a[0] + 1) * mj * mk;  // at most 512^3
+    for (int e = lane; e < cells; e += 32) {
+        const int i = a[0] + e / (mj * mk), j = a[1] + e / mk % mj, k = a[2] + e % mk;
         const size_t c = ((size_t)i * n1 + j) * n2 + k;
         if (!starts) {
             atomicAdd(&counts[c], 1);
