@@ -602,7 +602,8 @@ __device__ __forceinline__ bool fx_out(uint32_t e20) { return e20 - FX_EMIN >= F
 // halves of a slot add up by a shuffle.  (One warp with a whole stencil a lane
 // needs 255 registers; at eight warps an SM the multiply-add chains were exposed
 // and the pass took 435 us on the two-circle sphere at dx 0.025.)  The rows'
-// weights are broadcast from shared memory.
+// weights are broadcast from shared memory.  347 us there now: 54 M of its 206 M warp
+// instructions are the multiply-adds, and half of the issue slots are used.
 constexpr int EX_ROWS = 8;
 __global__ void __launch_bounds__(128, 5) k_epass32x(OpView<double> op, const Slot *sl, int ph, int nb_plain,
                                                      const double *x, double *t) {
@@ -932,7 +933,8 @@ __global__ void __launch_bounds__(E1_T, 7) k_epass1(OpView<T> op, const Slot *sl
     if (rows) {  // while the previous kernel ends
         e1_tables(op, c, lane, q);
         // the run's weights (a line a lane) on their way from DRAM while the values are
-        // gathered: 101.3 -> 92.4 us an apply on the torus at dx 0.01
+        // gathered: 101.3 -> 92.4 us an apply on the torus at dx 0.01 (98.7 since the sums
+        // keep two bits more)
         if (sizeof(T) == 8 && lane < ((q.ch.w & 255) * 96 + 127) / 128)
             asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)(op.w_fix + 12 * (int64_t)q.ch.y) + 128 * lane));
     }
@@ -988,8 +990,9 @@ static void slot_epatch(const OpView<T> &op, const Slot *sl, int ph, const T *x,
 // E_GROUPS groups.  FP32 apply at 8 / 16 / 32 / 64: two-circle sphere at dx 0.025
 // (27 thousand groups, 6 a warp at 8) 75.3 / 75.5 / 78.6 / 80.1 us, torus at 0.01
 // (222 thousand, 6 a warp at 64) 469 / 432 / 417 / 407 us; FP64 on the sphere (6 a
-// pair of warps at 16) 390 / 386 / 391 / 399 us.  The passes over groups with moved
-// columns do not mind.
+// pair of warps at 16) 390 / 386 / 391 / 399 us (410 at 16 since the sums keep two bits
+// more, and still the autotuner's choice).  The passes over groups with moved columns
+// do not mind.
 constexpr int E_GROUPS = 8, E_BPS_MIN = 8, E_BPS_MAX = 64, PATCH_BPS = 64;
 
 // groups a block takes at once: four warps with one (FP32) or two pairs (FP64)
